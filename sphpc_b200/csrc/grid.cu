@@ -251,284 +251,371 @@ __device__ __forceinline__ bool axis_regular(double x, double h, int c, int nmax
   return okm && okp;
 }
 
-struct BuildCtx {
-  float4 xf;              // x* as FP32 (candidate pre-test)
-  float4 xp, dp;          // exact representation x + d
-  double xs, ys, zs;      // canonical double x*
-  float h2lo, h2hi;
-  double h2d;
-};
-
 // r^2 < h^2 exactly as neighbors.c:278-285 evaluates it on the canonical
-// double positions.  The FP32 absolute positions decide every pair whose r^2
-// lies outside the band [P.bld_h2lo, P.bld_h2hi] = h^2 (1 -+ 2^-10); the FP64
-// test decides the rest.  The host opens the band to every pair when FP32
-// rounding of the grid's largest coordinate could move r^2 by that much
-// (sphpc_neighbor_pretest_fp32_safe: beyond about 2^12 h).
-__device__ __forceinline__ bool exact_neighbor(const BuildCtx& c, const PD* __restrict__ pd,
-                                            int j) {
-  float4 xq, dq;
+// double positions of slots p and j.  The FP32 absolute positions decide every
+// pair whose r^2 lies outside the band [P.bld_h2lo, P.bld_h2hi] = h^2 (1 -+
+// 2^-10); this test decides the rest.  The host opens the band to every pair
+// when FP32 rounding of the grid's largest coordinate could move r^2 by that
+// much (sphpc_neighbor_pretest_fp32_safe: beyond about 2^12 h).
+__device__ __forceinline__ bool exact_neighbor(const DevParams& P, const PD* __restrict__ pd,
+                                               int p, int j) {
+  float4 xp, dp, xq, dq;
+  ld_pd(pd, p, xp, dp);
   ld_pd(pd, j, xq, dq);
-  const double ddx = __dsub_rn(c.xs, xstar_d(xq.x, dq.x));
-  const double ddy = __dsub_rn(c.ys, xstar_d(xq.y, dq.y));
-  const double ddz = __dsub_rn(c.zs, xstar_d(xq.z, dq.z));
+  const double ddx = __dsub_rn(xstar_d(xp.x, dp.x), xstar_d(xq.x, dq.x));
+  const double ddy = __dsub_rn(xstar_d(xp.y, dp.y), xstar_d(xq.y, dq.y));
+  const double ddz = __dsub_rn(xstar_d(xp.z, dp.z), xstar_d(xq.z, dq.z));
   const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)),
                               __dmul_rn(ddz, ddz));
-  return r2 < c.h2d;
-}
-
-__device__ __forceinline__ bool is_neighbor(const BuildCtx& c, const PD* __restrict__ pd,
-                                            const float4* __restrict__ xsa, int j) {
-  const float4 q = xsa_load(xsa, j);
-  const float fx = c.xf.x - q.x, fy = c.xf.y - q.y, fz = c.xf.z - q.z;
-  const float r2f = norm2(fx, fy, fz);
-  if (r2f < c.h2lo) return true;
-  if (r2f > c.h2hi) return false;
-  return exact_neighbor(c, pd, j);
-}
-
-// Address of list entry t of particle p in the four-entry blocks nbr4[15][n].
-__device__ __forceinline__ size_t nbr_index(int n, int p, int t) {
-  return (((size_t)(t >> 2) * n + p) << 2) + (t & 3);
+  return r2 < P.h2d;
 }
 
 // FillNeighbors' 27-cell walk (neighbors.c:247-295) verbatim, for a
 // particle whose neighbour cells are not cx-1..cx+1 (FP64 rounding at a cell
 // face): its bucket goes to list entries 0..count-1 of p in nbr, the last
 // block's entries past the count are set to p; returns the count.
-__device__ __forceinline__ int walk_27_cells(const DevParams& P, const NbrView& V, const BuildCtx& c,
-                                          const PD* __restrict__ pd,
-                                          const float4* __restrict__ xsa, int p,
-                                          uint32_t* __restrict__ nbr) {
+__device__ __forceinline__ int walk_27_cells(const DevParams& P, const NbrView& V,
+                                             const PD* __restrict__ pd,
+                                             const float4* __restrict__ xsa, int p,
+                                             uint32_t* __restrict__ nbr) {
+  const float4 xf = xsa_load(xsa, p);
+  float4 xp, dp;
+  ld_pd(pd, p, xp, dp);
+  const double xs = xstar_d(xp.x, dp.x), ys = xstar_d(xp.y, dp.y), zs = xstar_d(xp.z, dp.z);
+  auto entry = [&](int t) -> uint32_t& { return nbr[(((size_t)(t >> 2) * V.n + p) << 2) + (t & 3)]; };
   int count = 0;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy)
       for (int dx = -1; dx <= 1; ++dx) {
         int gx, gy, gz;
-        if (!shifted_coord(__dadd_rn(c.xs, (double)dx * P.hd), P.hd, P.nx, gx)) continue;
-        if (!shifted_coord(__dadd_rn(c.ys, (double)dy * P.hd), P.hd, P.ny, gy)) continue;
-        if (!shifted_coord(__dadd_rn(c.zs, (double)dz * P.hd), P.hd, P.nz, gz)) continue;
+        if (!shifted_coord(__dadd_rn(xs, (double)dx * P.hd), P.hd, P.nx, gx)) continue;
+        if (!shifted_coord(__dadd_rn(ys, (double)dy * P.hd), P.hd, P.ny, gy)) continue;
+        if (!shifted_coord(__dadd_rn(zs, (double)dz * P.hd), P.hd, P.nz, gz)) continue;
         const uint32_t key = (uint32_t)P.nx * (uint32_t)P.ny * (uint32_t)gz +
                              ((uint32_t)gy * (uint32_t)P.nx + (uint32_t)gx);
         if (key >= P.ncells) continue;
         const int b = (int)__ldg(V.cstart + key);
         const int e = (int)__ldg(V.cstart + key + 1);
         for (int j = b; j < e && count < kMaxNeighbors; ++j) {
-          if (j != p && is_neighbor(c, pd, xsa, j)) nbr[nbr_index(V.n, p, count++)] = (uint32_t)j;
+          if (j == p) continue;
+          const float4 q = xsa_load(xsa, j);
+          const float r2 = norm2(xf.x - q.x, xf.y - q.y, xf.z - q.z);
+          if (r2 < P.bld_h2lo || (r2 <= P.bld_h2hi && exact_neighbor(P, pd, p, j)))
+            entry(count++) = (uint32_t)j;
         }
       }
-  for (int t = count; t & 3; ++t) nbr[nbr_index(V.n, p, t)] = (uint32_t)p;
+  for (int t = count; t & 3; ++t) entry(t) = (uint32_t)p;
   return count;
 }
 
 // ---------------------------------------------------------------------------
-// Staged neighbour build (FillNeighbors, neighbors.c:217-298): one thread per
+// Neighbour build (FillNeighbors, neighbors.c:217-298): one thread per
 // particle walks its 9 (dz, dy) slot rows in the reference's order (rows of
 // cells cx-1..cx+1 are contiguous slot ranges, cells in dx order, particles
 // in ascending original index), appending every candidate without branches
 // to its own column of a shared-memory staging area -- store the entry,
-// advance the count on a hit; the particle itself is skipped by splitting
-// its own row -- and writes its bucket out at the end as four-entry blocks
-// of nbr4[15][n] (for each block index, a warp's 32 consecutive slots are
+// advance the count on a hit -- and writes its bucket out at the end as
+// 16-byte blocks (for each block index, a warp's 32 consecutive slots are
 // four whole 128-byte lines), the last block's entries past the count set to
-// p.  A staged entry is 2 bytes, (row << 12) | offset in the
-// row, with the row starts kept in shared memory, so a thread holds 156
-// bytes of shared memory and the candidate loop only the particle's FP32
-// position: enough blocks stay resident to hide the candidate loads.  The
-// candidates of a row are tested two at a time with the packed FP32x2
-// arithmetic of sm_100 (staged_range).  A particle with a row of more than
-// 4095 candidates takes the verbatim 27-cell walk.
+// the particle itself.
+//
+// The candidates of a block of kTileSlots slots come from its tile of FP32
+// positions in shared memory (TileInfo; nine bulk copies), pairs of slots as
+// the 64-bit operands of the packed FP32x2 arithmetic of sm_100, and a staged
+// entry is the candidate's byte offset in the record tile, which is also the
+// list's entry.  A block whose tile does not fit loads the pairs from global
+// memory and stages (row << 12) | offset in the row, with the row starts in
+// shared memory.  A particle with a row of more than 4095 candidates takes the
+// verbatim 27-cell walk.
+//
+// Bounds: instruction issue (71%) and the shared-memory pipe (74%) together,
+// at five blocks per SM.  16.7M particles: 4024 us with every candidate pair
+// loaded per lane from global memory (the L1 data pipe at 88%), 3394 us so.
+// Tried for the same work and slower: the candidates of a cell held by a
+// warp's lanes, its particles broadcast to them and the hits taken from
+// ballots (240 warp instructions a particle against 136; 4.2M particles: 1462
+// us against 848).
 // ---------------------------------------------------------------------------
-constexpr int kStagedBlock = 128;
 constexpr int kRowBits = 12;
 constexpr int kRowMax = (1 << kRowBits) - 1;
+constexpr int kStageRows = kMaxNeighbors + 4;  // four candidates are appended at a time
 
-// Exact FP64 test of neighbors.c:278-285 for particle p and candidate j
-// (rare: only pairs whose FP32 r^2 lies in the band); reloads both records.
-__device__ __forceinline__ bool staged_exact(const DevParams& P, const PD* __restrict__ pd, int p,
-                                          int j) {
-  float4 xp, dpp, xq, dq;
-  ld_pd(pd, p, xp, dpp);
-  ld_pd(pd, j, xq, dq);
-  const double ddx = __dsub_rn(xstar_d(xp.x, dpp.x), xstar_d(xq.x, dq.x));
-  const double ddy = __dsub_rn(xstar_d(xp.y, dpp.y), xstar_d(xq.y, dq.y));
-  const double ddz = __dsub_rn(xstar_d(xp.z, dpp.z), xstar_d(xq.z, dq.z));
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)),
-                              __dmul_rn(ddz, ddz));
-  return r2 < P.h2d;
+// Whether the neighbour cells of a particle with FP32 position x in cell c of
+// an axis are c-1, c, c+1 (axis_regular) for certain: x / h lies at least
+// (c + 2) 2^-21 inside the cell, more than the FP32 rounding of x and of the
+// quotient, (c + 2) 2^-22, plus any FP64 rounding of (x +- h) / h.
+__device__ __forceinline__ bool axis_inside(float x, float inv_h, int c) {
+  const float f = fmaf(x, inv_h, -(float)c), m = (float)(c + 2) * 0x1p-21f;
+  return f > m && f < 1.0f - m;
 }
 
-// Test and append of one candidate slot j with FP32 r^2 = r2 (the exact
-// FP64 test decides inside the band): the entry is stored at the thread's
-// next staging slot and the count advances on a hit.
-__device__ __forceinline__ void staged_one(const DevParams& P, const PD* __restrict__ pd, int p,
-                                           int j, float r2, uint32_t entry,
+struct BuildRow {
+  const DevParams& P;
+  const PD* __restrict__ pd;
+  uint64_t pxx, pyy, pzz, mh2;
+  int p;
+};
+
+// Tests and appends candidates j .. j+3 (j even) of the range [lo, hi): with
+// MASK those outside it, and `skip`, are left out.  `slot` - j is the slot of
+// index 0.  s = r^2 - h^2 by fused multiply-adds from -h^2: its sign decides,
+// and the exact FP64 test where |s| lies in the band (the three roundings of
+// s stay within the bound that the band was sized for: near the band every
+// partial sum is at most h^2).
+template <bool TILE, bool MASK>
+__device__ __forceinline__ void build_four(const BuildRow& c, const float4* __restrict__ src, int j,
+                                           int lo, int hi, int skip, int dslot, uint32_t entry,
                                            uint16_t* __restrict__ stg, int& cnt) {
-  bool hit = r2 <= P.bld_h2hi;
-  if (hit && r2 >= P.bld_h2lo) hit = staged_exact(P, pd, p, j);
-  stg[cnt * kStagedBlock] = (uint16_t)entry;
-  cnt += hit ? 1 : 0;
-}
-
-// Test and append of the four candidates j .. j+3 with FP32 r^2 = r2[u]:
-// one branch for the group, taken only when a candidate lies in the band
-// (the exact FP64 test then decides those), then four branch-free appends.
-__device__ __forceinline__ void staged_four(const DevParams& P, const PD* __restrict__ pd, int p,
-                                            int j, const float (&r2)[4], uint32_t entry,
-                                            uint16_t* __restrict__ stg, int& cnt) {
-  bool hit[4];
-  bool band = false;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    hit[u] = r2[u] <= P.bld_h2hi;
-    band |= hit[u] && r2[u] >= P.bld_h2lo;
+  uint64_t x0, y0, z0, x1, y1, z1;
+  if (TILE) {
+    const ulonglong2* t = reinterpret_cast<const ulonglong2*>(src + j);
+    const ulonglong2 a = t[0], b = t[2];
+    x0 = a.x;
+    y0 = a.y;
+    x1 = b.x;
+    y1 = b.y;
+    z0 = *reinterpret_cast<const uint64_t*>(t + 1);
+    z1 = *reinterpret_cast<const uint64_t*>(t + 3);
+  } else {
+    ld_pair(src, j, x0, y0, z0);
+    ld_pair(src, j + 2, x1, y1, z1);
   }
-  if (band) {
+  uint64_t d = f2_sub(c.pxx, x0);
+  uint64_t s0 = f2_fma(d, d, c.mh2);
+  d = f2_sub(c.pyy, y0);
+  s0 = f2_fma(d, d, s0);
+  d = f2_sub(c.pzz, z0);
+  s0 = f2_fma(d, d, s0);
+  d = f2_sub(c.pxx, x1);
+  uint64_t s1 = f2_fma(d, d, c.mh2);
+  d = f2_sub(c.pyy, y1);
+  s1 = f2_fma(d, d, s1);
+  d = f2_sub(c.pzz, z1);
+  s1 = f2_fma(d, d, s1);
+  float s[4] = {f2_lo(s0), f2_hi(s0), f2_lo(s1), f2_hi(s1)};
+  const float band = c.P.bld_band;
+  auto inside = [&](int u) {
+    return (unsigned)(j + u - lo) < (unsigned)(hi - lo) && j + u != skip;
+  };
+  if (MASK) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = inside(u) ? s[u] : 3.0e38f;
+  }
+  const float m = fminf(fminf(fabsf(s[0]), fabsf(s[1])), fminf(fabsf(s[2]), fabsf(s[3])));
+  if (m <= band) {
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (hit[u] && r2[u] >= P.bld_h2lo) hit[u] = staged_exact(P, pd, p, j + u);
+      if (fabsf(s[u]) <= band && (!MASK || inside(u)))
+        s[u] = exact_neighbor(c.P, c.pd, c.p, j + u + dslot) ? -1.0f : 1.0f;
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    stg[cnt * kStagedBlock] = (uint16_t)(entry + u);
-    cnt += hit[u] ? 1 : 0;
+    stg[cnt * kTileSlots] = (uint16_t)(entry + (TILE ? 16 * u : u));
+    cnt += s[u] < 0.0f ? 1 : 0;
   }
 }
 
-// r^2 of one slot from the FP32 positions (the ragged ends of a range).
-__device__ __forceinline__ float staged_r2(const float4* __restrict__ xsa, int j, float px,
-                                           float py, float pz) {
-  const float4 q = xsa_load(xsa, j);
-  const float fx = px - q.x, fy = py - q.y, fz = pz - q.z;
-  return norm2(fx, fy, fz);
+// Appends the candidates [lo, hi) of one row except `skip` (< 0: none).
+template <bool TILE, bool SKIP>
+__device__ __forceinline__ void build_range(const BuildRow& c, const float4* __restrict__ src,
+                                            int lo, int hi, int skip, int dslot, uint32_t tag,
+                                            uint16_t* __restrict__ stg, int& cnt) {
+  if (lo >= hi || cnt >= kMaxNeighbors) return;
+  // (the first group may start one slot before lo: its offset -1 is not taken)
+  auto entry = [&](int j) {
+    return TILE ? (uint32_t)j << 4 : (tag << kRowBits) + (uint32_t)(j - lo);
+  };
+  int j = lo & ~1;
+  build_four<TILE, true>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
+  j += 4;
+  for (; j + 4 <= hi && cnt < kMaxNeighbors; j += 4)
+    build_four<TILE, SKIP>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
+  if (j < hi && cnt < kMaxNeighbors)
+    build_four<TILE, true>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
 }
 
-// Appends the candidates of slots [ja, jb) of row r (starting at slot rb),
-// entries (r << kRowBits) | (j - rb).  The slots of an even-aligned pair are
-// tested together with packed FP32x2 arithmetic (each lane rounds as the
-// scalar form would: x_p - x_q, then (dx^2 + dy^2) + dz^2 by fused
-// multiply-adds), two pairs per batch while four more entries fit below the
-// cap; an odd first or last slot is tested alone.
-__device__ __forceinline__ void staged_range(const DevParams& P, const PD* __restrict__ pd,
-                                             const float4* __restrict__ xsa, uint64_t pxx,
-                                             uint64_t pyy, uint64_t pzz, float px, float py,
-                                             float pz, int p, int r, int rb, int ja, int jb,
-                                             uint16_t* __restrict__ stg, int& cnt) {
-  const uint32_t tag = (uint32_t)r << kRowBits;
-  int j = ja;
-  if ((j & 1) && j < jb && cnt < kMaxNeighbors) {
-    staged_one(P, pd, p, j, staged_r2(xsa, j, px, py, pz), tag | (uint32_t)(j - rb), stg, cnt);
-    ++j;
-  }
-  for (; j + 4 <= jb && cnt <= kMaxNeighbors - 4; j += 4) {
-    // pair blocks of slots j, j+1 and j+2, j+3
-    uint64_t x0, y0, z0, x1, y1, z1;
-    ld_pair(xsa, j, x0, y0, z0);
-    ld_pair(xsa, j + 2, x1, y1, z1);
-    uint64_t d = f2_sub(pxx, x0);
-    uint64_t s0 = f2_mul(d, d);
-    d = f2_sub(pyy, y0);
-    s0 = f2_fma(d, d, s0);
-    d = f2_sub(pzz, z0);
-    s0 = f2_fma(d, d, s0);
-    d = f2_sub(pxx, x1);
-    uint64_t s1 = f2_mul(d, d);
-    d = f2_sub(pyy, y1);
-    s1 = f2_fma(d, d, s1);
-    d = f2_sub(pzz, z1);
-    s1 = f2_fma(d, d, s1);
-    const float r2[4] = {f2_lo(s0), f2_hi(s0), f2_lo(s1), f2_hi(s1)};
-    staged_four(P, pd, p, j, r2, tag | (uint32_t)(j - rb), stg, cnt);
-  }
-  for (; j + 2 <= jb && cnt <= kMaxNeighbors - 2; j += 2) {
-    uint64_t x0, y0, z0;
-    ld_pair(xsa, j, x0, y0, z0);
-    uint64_t d = f2_sub(pxx, x0);
-    uint64_t s0 = f2_mul(d, d);
-    d = f2_sub(pyy, y0);
-    s0 = f2_fma(d, d, s0);
-    d = f2_sub(pzz, z0);
-    s0 = f2_fma(d, d, s0);
-    const uint32_t e = tag | (uint32_t)(j - rb);
-    staged_one(P, pd, p, j, f2_lo(s0), e, stg, cnt);
-    staged_one(P, pd, p, j + 1, f2_hi(s0), e + 1, stg, cnt);
-  }
-  for (; j < jb && cnt < kMaxNeighbors; ++j)
-    staged_one(P, pd, p, j, staged_r2(xsa, j, px, py, pz), tag | (uint32_t)(j - rb), stg, cnt);
-}
-
-// 9 blocks of 128 threads per SM: 56 registers (8 bytes spilled since the
-// four-entry write-out, no slower at 16.7M particles than without; a tighter
-// cap spills more and gains nothing).
-__global__ void __launch_bounds__(kStagedBlock, 9)
-    k_build_staged(const DevParams P, const NbrView V, const PD* __restrict__ pd,
-                   const float4* __restrict__ xsa, const uint32_t* __restrict__ cellp,
-                   uint32_t* __restrict__ nbr, uint8_t* __restrict__ ncount) {
-  __shared__ uint16_t s_stage[kMaxNeighbors * kStagedBlock];
-  __shared__ int s_rowb[9 * kStagedBlock];
-  const int p = blockIdx.x * kStagedBlock + threadIdx.x;
-  if (p >= P.n) return;
-  uint16_t* stg = s_stage + threadIdx.x;
-  int* rowb = s_rowb + threadIdx.x;
-  BuildCtx c;
-  ld_pd(pd, p, c.xp, c.dp);
-  c.xs = xstar_d(c.xp.x, c.dp.x);
-  c.ys = xstar_d(c.xp.y, c.dp.y);
-  c.zs = xstar_d(c.xp.z, c.dp.z);
+// The nine rows of particle p, tile: src is the tile and off[r] = o[r] - s[r]
+// takes slots to tile records; else src is xsa and rowb receives the row
+// starts (stride kTileSlots).  Returns the staged count, at most
+// kMaxNeighbors, or -1 for a row beyond kRowMax (without a tile).
+template <bool TILE>
+__device__ __forceinline__ int build_rows(const BuildRow& c, const NbrView& V, uint32_t cell,
+                                          const float4* __restrict__ src, const int* off,
+                                          int* rowb, uint16_t* __restrict__ stg) {
+  const DevParams& P = c.P;
   int cx, cy, cz;
-  unpack_cell(V, __ldg(cellp + p), cx, cy, cz);
-  bool regular = axis_regular(c.xs, P.hd, cx, P.nx) && axis_regular(c.ys, P.hd, cy, P.ny) &&
-                 axis_regular(c.zs, P.hd, cz, P.nz);
-  // the 9 rows' slot ranges (empty outside the grid)
-  const int xlo = cx - (cx > 0);
-  const int xhi = cx + (cx < P.nx - 1);
-  if (regular) {
+  unpack_cell(V, cell, cx, cy, cz);
+  const int xlo = cx - (cx > 0), xhi = cx + (cx < P.nx - 1) + 1;
+  auto bounds = [&](int r, int& b, int& e) {
+    const int z = cz + r / 3 - 1, y = cy + r % 3 - 1;
+    b = e = 0;
+    if (r < 9 && (unsigned)z < (unsigned)P.nz && (unsigned)y < (unsigned)P.ny) {
+      const uint32_t rk = (uint32_t)z * P.nxny + (uint32_t)y * (uint32_t)P.nx;
+      b = (int)__ldg(V.cstart + rk + xlo);
+      e = (int)__ldg(V.cstart + rk + xhi);
+    }
+  };
+  if (!TILE) {
     for (int r = 0; r < 9; ++r) {
-      const int z = cz + r / 3 - 1, y = cy + r % 3 - 1;
-      int b = 0, e = 0;
-      if ((unsigned)z < (unsigned)P.nz && (unsigned)y < (unsigned)P.ny) {
-        const uint32_t rk = (uint32_t)z * P.nxny + (uint32_t)y * (uint32_t)P.nx;
-        b = (int)__ldg(V.cstart + rk + xlo);
-        e = (int)__ldg(V.cstart + rk + xhi + 1);
-      }
-      if (e - b > kRowMax) regular = false;  // the row offset would not fit
-      rowb[r * kStagedBlock] = b;
+      int b, e;
+      bounds(r, b, e);
+      if (e - b > kRowMax) return -1;
     }
   }
-  int count = 0;
-  if (regular) {
-    const float4 xf = xsa_load(xsa, p);
-    const uint64_t pxx = f2_dup(xf.x), pyy = f2_dup(xf.y), pzz = f2_dup(xf.z);
-    for (int r = 0; r < 9 && count < kMaxNeighbors; ++r) {
-      const int z = cz + r / 3 - 1, y = cy + r % 3 - 1;
-      if ((unsigned)z >= (unsigned)P.nz || (unsigned)y >= (unsigned)P.ny) continue;
-      const uint32_t rk = (uint32_t)z * P.nxny + (uint32_t)y * (uint32_t)P.nx;
-      const int b = rowb[r * kStagedBlock];
-      const int e = (int)__ldg(V.cstart + rk + xhi + 1);
-      if (r == 4) {
-        staged_range(P, pd, xsa, pxx, pyy, pzz, xf.x, xf.y, xf.z, p, r, b, b, p, stg, count);
-        staged_range(P, pd, xsa, pxx, pyy, pzz, xf.x, xf.y, xf.z, p, r, b, p + 1, e, stg, count);
-      } else {
-        staged_range(P, pd, xsa, pxx, pyy, pzz, xf.x, xf.y, xf.z, p, r, b, b, e, stg, count);
+  int cnt = 0, b, e;
+  bounds(0, b, e);
+  for (int r = 0; r < 9; ++r) {
+    int bn, en;
+    bounds(r + 1, bn, en);  // the next row's, ahead of this row's tests
+    const int o = TILE ? off[r] : 0;
+    if (!TILE) rowb[r * kTileSlots] = b;
+    if (r == 4)
+      build_range<TILE, true>(c, src, b + o, e + o, c.p + o, -o, (uint32_t)r, stg, cnt);
+    else
+      build_range<TILE, false>(c, src, b + o, e + o, -1, -o, (uint32_t)r, stg, cnt);
+    b = bn;
+    e = en;
+  }
+  return min(cnt, kMaxNeighbors);
+}
+
+// The nine ranges of the block's tile (TileInfo): computed by lanes 0..8 of
+// warp 0 into t.
+__device__ __forceinline__ void tile_ranges(const DevParams& P, const NbrView& V,
+                                            const uint32_t* __restrict__ cellp, int first,
+                                            int last, TileInfo& t) {
+  const int r = threadIdx.x;
+  int s = 0, len = 0;
+  if (r < 9) {
+    int cx, cy, cz;
+    unpack_cell(V, __ldg(cellp + first), cx, cy, cz);
+    const int64_t k0 = (int64_t)cell_key(P, cx, cy, cz);
+    unpack_cell(V, __ldg(cellp + last), cx, cy, cz);
+    const int64_t k1 = (int64_t)cell_key(P, cx, cy, cz);
+    const int64_t d = (int64_t)(r / 3 - 1) * P.nxny + (int64_t)(r % 3 - 1) * P.nx;
+    const int64_t lo = min(max(k0 + d - 1, (int64_t)0), (int64_t)P.ncells);
+    const int64_t hi = min(max(k1 + d + 2, (int64_t)0), (int64_t)P.ncells);
+    s = (int)__ldg(V.cstart + lo) & ~1;
+    len = (((int)__ldg(V.cstart + hi) + 1) & ~1) - s;
+    len = max(len, 0);
+  }
+  int o = len;
+#pragma unroll
+  for (int k = 1; k < 16; k <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, o, k);
+    if (r >= k) o += y;
+  }
+  if (r < 9) {
+    t.s[r] = s;
+    t.o[r] = o - len;
+  }
+  if (r == 8) t.total = o;
+}
+
+// Staging column of a thread: halfwords of warps 2k and 2k + 1 share a 32-bit
+// word, so a warp's 32 columns lie in 32 banks whatever their counts.
+__device__ __forceinline__ int stage_column() {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  return ((warp >> 1) * 32 + lane) * 2 + (warp & 1);
+}
+
+// Five blocks of 128 threads per SM with their tiles (40 KB).
+__global__ void __launch_bounds__(kTileSlots, 5)
+    k_build(const DevParams P, const NbrView V, const PD* __restrict__ pd,
+            const float4* __restrict__ xsa, const uint32_t* __restrict__ cellp,
+            uint32_t* __restrict__ nbr, uint8_t* __restrict__ ncount, TileInfo* __restrict__ tiles) {
+  // the tile (its last group of four may read three records past it), or the
+  // row starts of a block without one
+  __shared__ __align__(128) float4 s_tile[kTileCap + 4];
+  __shared__ uint16_t s_stage[kStageRows * kTileSlots];
+  __shared__ TileInfo s_info;
+  __shared__ int s_off[9];
+  __shared__ __align__(8) uint64_t s_mbar;
+  const int first = blockIdx.x * kTileSlots;
+  const int p = first + threadIdx.x;
+  const bool own = p < P.n;
+  uint32_t cell = 0;
+  bool regular = true;
+  float4 xf = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (own) {
+    xf = xsa_load(xsa, p);
+    cell = __ldg(cellp + p);
+    int cx, cy, cz;
+    unpack_cell(V, cell, cx, cy, cz);
+    const float inv_h = 1.0f / P.h;
+    if (!(axis_inside(xf.x, inv_h, cx) && axis_inside(xf.y, inv_h, cy) &&
+          axis_inside(xf.z, inv_h, cz))) {
+      float4 xp, dp;
+      ld_pd(pd, p, xp, dp);
+      regular = axis_regular(xstar_d(xp.x, dp.x), P.hd, cx, P.nx) &&
+                axis_regular(xstar_d(xp.y, dp.y), P.hd, cy, P.ny) &&
+                axis_regular(xstar_d(xp.z, dp.z), P.hd, cz, P.nz);
+    }
+  }
+  if (threadIdx.x < 32) tile_ranges(P, V, cellp, first, min(first + kTileSlots, P.n) - 1, s_info);
+  const bool all_regular = __syncthreads_and(regular ? 1 : 0) != 0;
+  const int total = s_info.total;
+  const bool tiled = all_regular && total <= kTileCap;
+  if (threadIdx.x < 32) {
+    const int r = threadIdx.x;
+    if (r < 9) {
+      s_off[r] = s_info.o[r] - s_info.s[r];
+      tiles[blockIdx.x].s[r] = s_info.s[r];
+      tiles[blockIdx.x].o[r] = s_info.o[r];
+    }
+    if (r == 9) tiles[blockIdx.x].total = tiled ? total : -1;
+    if (tiled) {
+      if (r == 0) {
+        mbar_init1(&s_mbar);
+        mbar_expect(&s_mbar, (uint32_t)total * 16u);
+      }
+      __syncwarp();
+      if (r < 9) {
+        const int o = s_info.o[r], e = r < 8 ? s_info.o[r + 1] : total;
+        if (e > o) bulk_load(s_tile + o, xsa + s_info.s[r], (uint32_t)(e - o) * 16u, &s_mbar);
       }
     }
-    // one 16-byte block of four entries per store; the last block's entries
-    // past the count are p
-    uint4* out = reinterpret_cast<uint4*>(nbr) + p;
-    auto entry = [&](int t) {
-      const uint32_t en = stg[t * kStagedBlock];
-      return t < count ? (uint32_t)(rowb[(en >> kRowBits) * kStagedBlock] + (int)(en & kRowMax))
-                       : (uint32_t)p;
-    };
+  }
+  __syncthreads();
+  if (tiled && !mbar_wait0(&s_mbar)) {
+    atomicOr(V.err, kErrTileWait);
+    mbar_wait0(&s_mbar);
+  }
+  if (!own) return;
+  uint16_t* stg = s_stage + stage_column();
+  const BuildRow c{P, pd, f2_dup(xf.x), f2_dup(xf.y), f2_dup(xf.z), f2_dup(-P.h2), p};
+  uint4* out = reinterpret_cast<uint4*>(nbr) + p;
+  int count;
+  if (tiled) {
+    count = build_rows<true>(c, V, cell, s_tile, s_off, nullptr, stg);
+    const uint32_t self = (uint32_t)(p + s_off[4]) << 4;
 #pragma unroll 1
-    for (int t0 = 0; t0 < count; t0 += 4, out += P.n)
-      *out = make_uint4(entry(t0), entry(t0 + 1), entry(t0 + 2), entry(t0 + 3));
+    for (int t0 = 0; t0 < count; t0 += 8, out += P.n) {
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = t0 + 2 * u;
+        const uint32_t a = t < count ? stg[t * kTileSlots] : self;
+        const uint32_t b = t + 1 < count ? stg[(t + 1) * kTileSlots] : self;
+        w[u] = a | (b << 16);
+      }
+      *out = make_uint4(w[0], w[1], w[2], w[3]);
+    }
   } else {
-    c.xf = xsa_load(xsa, p);
-    c.h2lo = P.bld_h2lo;
-    c.h2hi = P.bld_h2hi;
-    c.h2d = P.h2d;
-    count = walk_27_cells(P, V, c, pd, xsa, p, nbr);
+    int* rowb = reinterpret_cast<int*>(s_tile) + threadIdx.x;
+    count = regular ? build_rows<false>(c, V, cell, xsa, nullptr, rowb, stg) : -1;
+    if (count < 0) {
+      count = walk_27_cells(P, V, pd, xsa, p, nbr);
+    } else {
+      auto entry = [&](int t) {
+        if (t >= count) return (uint32_t)p;
+        const uint32_t en = stg[t * kTileSlots];
+        return (uint32_t)(rowb[(en >> kRowBits) * kTileSlots] + (int)(en & kRowMax));
+      };
+#pragma unroll 1
+      for (int t0 = 0; t0 < count; t0 += 4, out += P.n)
+        *out = make_uint4(entry(t0), entry(t0 + 1), entry(t0 + 2), entry(t0 + 3));
+    }
   }
   ncount[p] = (uint8_t)count;
 }
@@ -541,17 +628,12 @@ __global__ void __launch_bounds__(kBlock)
   if (p >= V.n) return;
   // the list's last block must hold p past the count (the batched visits
   // read those entries as the pair (p, p))
-  const int c0 = (int)__ldg(V.ncount + p);
-  for (int t = c0; t & 3; ++t)
+  const int cnt = (int)__ldg(V.ncount + p), per = has_tile(V, p) ? 8 : 4;
+  for (int t = cnt; t & (per - 1); ++t)
     if (nbr_entry(V, p, t) != (uint32_t)p) atomicOr(err, kErrNbrTail);
   const uint32_t idp = __ldg(ids + p);
   uint32_t* out = nbr + (size_t)idp * kMaxNeighbors;
-  int cnt = 0;
-  for_each_neighbor(V, p, [&](int q) {
-    if (cnt < kMaxNeighbors) out[cnt] = __ldg(ids + q);
-    ++cnt;
-  });
-  for (int j = cnt; j < kMaxNeighbors; ++j) out[j] = 0u;
+  for (int j = 0; j < kMaxNeighbors; ++j) out[j] = j < cnt ? __ldg(ids + nbr_entry(V, p, j)) : 0u;
   count[idp] = cnt;
 }
 
@@ -590,9 +672,9 @@ void launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uin
 
 void launch_build_neighbors(const DevParams& P, const NbrView& V, const PD* pd,
                             const float4* xsa, const uint32_t* cellp, uint32_t* nbr,
-                            uint8_t* ncount, cudaStream_t st) {
-  k_build_staged<<<grid_for(P.n, kStagedBlock), kStagedBlock, 0, st>>>(P, V, pd, xsa, cellp, nbr,
-                                                                        ncount);
+                            uint8_t* ncount, TileInfo* tiles, cudaStream_t st) {
+  k_build<<<grid_for(P.n, kTileSlots), kTileSlots, 0, st>>>(P, V, pd, xsa, cellp, nbr, ncount,
+                                                            tiles);
 }
 
 void launch_export_buckets(const NbrView& V, const uint32_t* ids, uint32_t* nbr, int32_t* count,

@@ -51,11 +51,11 @@ void launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uin
                         uint4* gaps, uint32_t* gap_count, uint32_t* err, cudaStream_t st);
 
 // Neighbour build (FillNeighbors, neighbors.c:217-298): per particle, its
-// bucket of neighbour slots (four-entry blocks nbr4[j / 4][p], entries past
-// the count in the last block set to p) and its size ncount[p].
+// bucket as blocks of list entries (sphpc_dev.cuh) and its size ncount[p], and
+// the tiles of its blocks (ceil(n / kTileSlots) entries).
 void launch_build_neighbors(const DevParams& P, const NbrView& V, const PD* pd,
                             const float4* xsa, const uint32_t* cellp, uint32_t* nbr,
-                            uint8_t* ncount, cudaStream_t st);
+                            uint8_t* ncount, TileInfo* tiles, cudaStream_t st);
 
 // Export the buckets in original-index space: nbr[id*60 + j], count[id];
 // raises kErrNbrTail in err if a list's last block does not hold p past the
@@ -84,8 +84,6 @@ struct PassArgs {
   float* lam_acc;      // position pass: multiplier applied so far this step,
                        // sum of stiffness * lambda_p (null: not kept)
   int acc_add;         // 1: add to lam_acc, 0: start it with this pass
-  const NV* nv;        // post passes: {record, colour or velocity} gathered
-  NV* nv_out;          // post passes: {record, colour or velocity} for the next pass
 };
 
 // Density (+lambda) pass: ComputeDensities (particles.c:461-514) and
@@ -111,23 +109,19 @@ void launch_position(const DevParams& P, const NbrView& V, const PassArgs& a, in
                      cudaStream_t st);
 // UpdatePositionStars alone, in place on pd_out: d += dp, clamp, SDF.
 void launch_apply_dp(const DevParams& P, const PassArgs& a, cudaStream_t st);
-// nv[p] = {nr[p], e[p]}: the combined records of a post pass whose
-// producer did not write them.
-void launch_pack_nv(int n, const uint4* nr, const float4* e, NV* nv, cudaStream_t st);
 // ComputeSurfaceTension colour pass (:94-140) and force pass (:142-204).
-// The colour pass gathers nr (neighbour densities in w) and writes color[]
-// and nv_out = {nr, colour}; the force pass gathers nv, updates vel in place
-// and, if nv_out is set, writes {nr, new velocity} there.
+// The colour pass gathers nr (neighbour densities in w) and writes color[];
+// the force pass gathers nr and color and updates vel in place.
 void launch_color(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st);
 void launch_tension(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st);
-// ApplyViscosity (:383-459) as a Jacobi update of the velocities in nv into
-// vel_out (and, if set, nv_out = {nr, new velocity}); with write_pos also
-// UpdatePositions into pd_out.
+// ApplyViscosity (:383-459) as a Jacobi update of vel into vel_out; with
+// write_pos also UpdatePositions into pd_out.
 void launch_xsph(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st);
-// ComputeVorticity (:207-283) from the velocities in nv;
-// ApplyVorticityConfinement (:285-381) updates vel in place.
+// ComputeVorticity (:207-283) from the velocities vel (with nr_out also the
+// records {X, |omega|}); ApplyVorticityConfinement (:285-381) gathers those
+// records and updates vel in place.
 void launch_vorticity(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st);
-void launch_confinement(const DevParams& P, const NbrView& V, const PassArgs& a, bool omega_in_nr,
+void launch_confinement(const DevParams& P, const NbrView& V, const PassArgs& a,
                         cudaStream_t st);
 // Pointwise steps.
 void launch_gravity(const DevParams& P, float4* vel, cudaStream_t st);
@@ -139,10 +133,10 @@ void launch_update_positions(const DevParams& P, PD* pd, cudaStream_t st);
 // d.w and/or the record payload <- src[p] (a per-particle scalar for the
 // neighbour passes; null pd or nr skips it).
 void launch_pack_w(const DevParams& P, PD* pd, uint4* nr, const float* src, cudaStream_t st);
-// Neighbour records from particle records: canonical x* and payload src[p]
-// (d.w when src is null).
+// Neighbour records from particle records: canonical x* and payload
+// src[p * stride] (d.w when src is null).
 void launch_make_nr(const DevParams& P, const PD* pd, const float* src, uint4* nr,
-                    cudaStream_t st);
+                    cudaStream_t st, int stride = 1);
 // CalculateParticleCollisions seam on device double arrays.
 void launch_collisions_double(const DevParams& P, double* x, double* y, double* z, int n,
                               cudaStream_t st);

@@ -1,12 +1,26 @@
 // pbf.cu -- the neighbour passes and pointwise steps of one PBF time step.
 //
 // Every pass is one thread per particle in slot (cell-sorted) order; the
-// neighbour loop visits the bucket of the particle in the reference's order
-// (for_each_neighbor).  Sums are FP32 (density with Kahan compensation);
-// the box clamp, the SDF lookup and the position update are FP64 on the
-// canonical double x* = x + d of the particle's own record.  Neighbours are
-// read from the 16-byte records (fixed-point x* and a payload) with one
-// 128-bit load each; the pair difference is their exact integer difference.
+// neighbour loop visits the bucket of the particle in the reference's order.
+// Sums are FP32 (density with Kahan compensation); the box clamp, the SDF
+// lookup and the position update are FP64 on the canonical double x* = x + d
+// of the particle's own record.  Neighbours are read from the 16-byte records
+// (fixed-point x* and a payload), and a vector beside them in the passes that
+// need one; the pair difference is their exact integer difference.
+//
+// A block of kTileSlots threads first brings the records of its neighbourhood
+// into shared memory (its tile, sphpc_dev.cuh: nine bulk copies, about 1400
+// records) and its lists index them; a block without a tile gathers from
+// global memory.
+//
+// Bounds: the shared-memory pipe (70-80% of its wavefronts).  A warp's gather
+// of 32 16-byte records costs about nine wavefronts (eight lanes at a time, a
+// conflict where two of them read different records of one 16-byte bank
+// group), where the same gather through the L1 touched thirteen 128-byte
+// lines, and a list entry takes two bytes instead of four.  At 16.7M
+// particles, per launch: density 917 -> 724 us, position 1048 -> 904, colour
+// and tension 2582 -> 2255, XSPH 1647 -> 1622, vorticity and confinement
+// 2585 -> 2442.
 #include "kernels.cuh"
 
 namespace sphpc {
@@ -17,28 +31,42 @@ struct Pair {
   float dx, dy, dz, r2;
 };
 
-// neighbours whose list entries and records are fetched together
-constexpr int kNbrBatch = 4;
-// resident 256-thread blocks per SM asked of the compiler for the neighbour
-// passes (register caps of 40, 48 and 64; more resident warps hide the gather
-// latency better than the registers a larger allocation would keep, as long
-// as the neighbour loop itself does not spill).  The position pass runs at 48:
-// at 40 its FP64 epilogue spills up to 88 bytes a thread through the L1 that
-// its gathers already keep busy (2.4-3.5% slower at 16.7M particles).
-constexpr int kMinBlocksDensity = 6;
-constexpr int kMinBlocksPosition = 5;
-constexpr int kMinBlocksColor = 5;
-constexpr int kMinBlocksVorticity = 5;
-constexpr int kMinBlocksConfinement = 6;
-constexpr int kMinBlocksTension = 4;  // 64 registers: at 48 the loop spills
-constexpr int kMinBlocksXsph = 4;
-constexpr int kMinBlocksFeatures = 4;
+// Resident blocks of kTileSlots threads asked of the compiler: one tile of
+// records (23.5 KB) fits nine times into an SM's shared memory, two four times.
+constexpr int kMinBlocks1 = 9;
+constexpr int kMinBlocks2 = 4;
+constexpr int kMinBlocksFeatures = 8;
 
-// x*_p - x*_q as (x_p - x_q) + (d_p - d_q): exact in the first term for any
-// box size, so the FP32 pair geometry keeps its relative precision.
+// Head of a neighbour pass: the particle, its list's size and first block, and
+// the start of the tile's copies (NARR arrays of records).
+#define SPHPC_PASS_HEAD(NARR, arr0, arr1)                                          \
+  extern __shared__ __align__(128) unsigned char tile[];                           \
+  __shared__ __align__(8) uint64_t s_mbar;                                         \
+  const bool tiled = tile_load<NARR>(V, arr0, arr1, tile, &s_mbar);                \
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;                             \
+  const bool own = p < P.n;                                                        \
+  int cnt = own ? (int)__ldg(V.ncount + p) : 0;                                    \
+  const uint4 blk = cnt > 0 ? nbr_block(V, p, 0) : make_uint4(0u, 0u, 0u, 0u)
+// Before the list is visited: the tile has arrived (a wait that gave up raises
+// its error bit and visits nothing).
+#define SPHPC_PASS_READY() \
+  if (!tile_wait(V, tiled, &s_mbar)) cnt = 0
+
 __device__ __forceinline__ void ld_rw(const PD* base, int i, float4& x, float4& d) {
   x = base[i].x;
   d = base[i].d;
+}
+
+// x*_p - x*_q as (x_p - x_q) + (d_p - d_q): exact in the first term for any
+// box size, so the FP32 pair geometry keeps its relative precision.
+__device__ __forceinline__ Pair pair_geom(const float4 xp, const float4 dp, const float4 xq,
+                                          const float4 dq) {
+  Pair g;
+  g.dx = (xp.x - xq.x) + (dp.x - dq.x);
+  g.dy = (xp.y - xq.y) + (dp.y - dq.y);
+  g.dz = (xp.z - xq.z) + (dp.z - dq.z);
+  g.r2 = norm2(g.dx, g.dy, g.dz);
+  return g;
 }
 
 // x*_p - x*_q from two 16-byte records: the wrapping integer difference is
@@ -52,21 +80,59 @@ __device__ __forceinline__ Pair pair_nr(const DevParams& P, const uint4 a, const
   return g;
 }
 
-__device__ __forceinline__ Pair pair_geom(const float4 xp, const float4 dp, const float4 xq,
-                                          const float4 dq) {
-  Pair g;
-  g.dx = (xp.x - xq.x) + (dp.x - dq.x);
-  g.dy = (xp.y - xq.y) + (dp.y - dq.y);
-  g.dz = (xp.z - xq.z) + (dp.z - dq.z);
-  g.r2 = norm2(g.dx, g.dy, g.dz);
-  return g;
+// Two neighbours' pair geometry at a time as packed FP32x2 values (low half:
+// the first neighbour): a packed operation is issued once for two neighbours
+// and rounds each as its scalar form; what a list's order fixes -- the running
+// sums -- stays scalar.  Kept where issue comes next after the shared-memory
+// pipe (4.2M particles, scalar -> packed: density 204 -> 190 us, position 241
+// -> 234); the passes that gather a vector too are no faster with it (tension
+// 581 -> 598, XSPH 409 -> 411, vorticity 620 -> 626) and stay scalar.
+//
+// Differences x*_p - x*_q of two 16-byte records in fixed-point units: the
+// wrapping integer difference is exact, its conversion to FP32 rounds like any
+// FP32 difference.
+struct Pair2 {
+  uint64_t x, y, z;
+};
+__device__ __forceinline__ Pair2 diff2(const uint4 p, const uint4 a, const uint4 b) {
+  return {f2_pack((float)(int)(p.x - a.x), (float)(int)(p.x - b.x)),
+          f2_pack((float)(int)(p.y - a.y), (float)(int)(p.y - b.y)),
+          f2_pack((float)(int)(p.z - a.z), (float)(int)(p.z - b.z))};
+}
+// |d|^2 of both, as norm2.
+__device__ __forceinline__ uint64_t norm2_2(const Pair2& d) {
+  return f2_fma(d.z, d.z, f2_fma(d.y, d.y, f2_mul(d.x, d.x)));
+}
+__device__ __forceinline__ uint64_t max2(uint64_t a, float b) {
+  return f2_pack(fmaxf(f2_lo(a), b), fmaxf(f2_hi(a), b));
+}
+
+// 1/sqrt(x) of a normal x (PTX rsqrt.approx.ftz.f32): the value rsqrtf gives,
+// without the range test and the two scalings that rsqrtf spends on subnormal
+// arguments, which the floors below rule out.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+__device__ __forceinline__ uint64_t rsqrt2(uint64_t a) {
+  return f2_pack(rsqrt_normal(f2_lo(a)), rsqrt_normal(f2_hi(a)));
 }
 
 // r_mag floored at 1e-4 h (particles.c:635-637): returns r and 1/r.
 __device__ __forceinline__ void floored_r(const DevParams& P, float r2, float& r, float& rinv) {
   const float r2c = fmaxf(r2, P.rmin * P.rmin);
-  rinv = rsqrtf(r2c);
+  rinv = rsqrt_normal(r2c);
   r = __fmul_rn(r2c, rinv);
+}
+
+// max(h - r, 0) of two neighbours in fixed-point units, from r^2 floored at
+// r_min^2 and its reciprocal root, one fused multiply-add each: r - h
+// (rounded as h - r), then the sign turned with the floor.
+__device__ __forceinline__ uint64_t h_minus_r(const DevParams& P, uint64_t r2c, uint64_t rinv) {
+  const uint64_t m = f2_fma(r2c, rinv, f2_dup(-P.h_fx));
+  return f2_pack(fmaxf(-f2_lo(m), 0.0f), fmaxf(-f2_hi(m), 0.0f));
 }
 
 // The same in fixed-point units (r2f = |d|^2 of the record difference):
@@ -76,7 +142,7 @@ __device__ __forceinline__ void floored_r(const DevParams& P, float r2, float& r
 __device__ __forceinline__ void floored_r_fx(const DevParams& P, float r2f, float& r2c,
                                              float& rinv) {
   r2c = fmaxf(r2f, P.rmin2_fx);
-  rinv = rsqrtf(r2c);
+  rinv = rsqrt_normal(r2c);
 }
 __device__ __forceinline__ float fx_r(float r2c, float rinv) { return __fmul_rn(r2c, rinv); }
 __device__ __forceinline__ float fx_hm(const DevParams& P, float r2c, float rinv) {
@@ -93,8 +159,8 @@ __device__ __forceinline__ float rcp_fast(float x) {
   return r;
 }
 
+// max and sum of the per-particle density error over the block (FP64).
 __device__ __forceinline__ void block_resid(double e, double* resid) {
-  // max and sum of the per-particle density error over the block (FP64).
   double m = e, s = e;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -110,7 +176,7 @@ __device__ __forceinline__ void block_resid(double e, double* resid) {
   __syncthreads();
   if (threadIdx.x == 0) {
     double bm = 0.0, bs = 0.0;
-    for (int w = 0; w < kBlock / 32; ++w) {
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) {
       bm = fmax(bm, sm[w]);
       bs += ss[w];
     }
@@ -121,12 +187,13 @@ __device__ __forceinline__ void block_resid(double e, double* resid) {
 }
 
 template <int MODE, bool RESID>
-__global__ void __launch_bounds__(kBlock, kMinBlocksDensity)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
     k_density_lambda(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  SPHPC_PASS_HEAD(1, a.nr, nullptr);
   double err = 0.0;
-  if (p < P.n) {
-    const uint4 rp = ld_nr(a.nr, p);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  SPHPC_PASS_READY();
+  if (own) {
     // The loop keeps only what varies per pair: the density sums t^3 with
     // t = h^2 - r^2 and the gradient sums c d with c = (h - r)^2 / r and d
     // the pair difference, both in fixed-point units; the kernel norms, the
@@ -138,40 +205,44 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksDensity)
     // terms carry d = 0.
     float st = 0.0f, comp = 0.0f;
     float sgx = 0.f, sgy = 0.f, sgz = 0.f, sC = 0.f;
-    for_each_batch_nr<kNbrBatch>(V, a.nr, p, [&](const uint4 (&rq)[kNbrBatch], int nvalid) {
-      float t3[kNbrBatch];
+    visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk,
+                    [&](const Batch<1>& q, int nvalid) {
+      float t[4], t2[4];
 #pragma unroll
-      for (int u = 0; u < kNbrBatch; ++u) {
-        const float fx = (float)(int)(rp.x - rq[u].x);
-        const float fy = (float)(int)(rp.y - rq[u].y);
-        const float fz = (float)(int)(rp.z - rq[u].z);
-        const float r2f = norm2(fx, fy, fz);
+      for (int u = 0; u < 4; u += 2) {
+        const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
+        const uint64_t r2f = norm2_2(d);
         if (MODE != 2) {
-          float t = fmaxf(fmaf(-P.fx_inv2, r2f, P.h2), 0.0f);
-          t = u < nvalid ? t : 0.0f;
-          t3[u] = t;
+          uint64_t tt = max2(f2_fma(f2_dup(-P.fx_inv2), r2f, f2_dup(P.h2)), 0.0f);
+          tt = f2_pack(u < nvalid ? f2_lo(tt) : 0.0f, u + 1 < nvalid ? f2_hi(tt) : 0.0f);
+          t[u] = f2_lo(tt);
+          t[u + 1] = f2_hi(tt);
+          tt = f2_mul(tt, tt);
+          t2[u] = f2_lo(tt);
+          t2[u + 1] = f2_hi(tt);
         }
         if (MODE != 1) {
           // in fixed-point units: c_f = (h_f - r_f)^2 / r_f = 2^k c
-          float r2c, rinv;
-          floored_r_fx(P, r2f, r2c, rinv);
-          const float hm = fx_hm(P, r2c, rinv);
-          const float c = __fmul_rn(__fmul_rn(hm, hm), rinv);
+          const uint64_t r2c = max2(r2f, P.rmin2_fx);
+          const uint64_t rinv = rsqrt2(r2c);
+          const uint64_t hm = h_minus_r(P, r2c, rinv);
+          const uint64_t c = f2_mul(f2_mul(hm, hm), rinv);
+          const uint64_t cc = f2_mul(c, c);
           // |c d|^2 = c^2 |d|^2: three fused accumulations and one for the norm
-          sgx = fmaf(c, fx, sgx);
-          sgy = fmaf(c, fy, sgy);
-          sgz = fmaf(c, fz, sgz);
-          sC = fmaf(__fmul_rn(c, c), r2f, sC);
+          sgx = fmaf(f2_lo(c), f2_lo(d.x), sgx);
+          sgy = fmaf(f2_lo(c), f2_lo(d.y), sgy);
+          sgz = fmaf(f2_lo(c), f2_lo(d.z), sgz);
+          sC = fmaf(f2_lo(cc), f2_lo(r2f), sC);
+          sgx = fmaf(f2_hi(c), f2_hi(d.x), sgx);
+          sgy = fmaf(f2_hi(c), f2_hi(d.y), sgy);
+          sgz = fmaf(f2_hi(c), f2_hi(d.z), sgz);
+          sC = fmaf(f2_hi(cc), f2_hi(r2f), sC);
         }
       }
       if (MODE != 2) {
-        static_assert(kNbrBatch == 4, "batch sum of four terms");
         // t0^3 + t1^3 + t2^3 + t3^3 as a chain of fused multiply-adds
-        const float* t = t3;
-        const float yb = fmaf(__fmul_rn(t[0], t[0]), t[0],
-                              fmaf(__fmul_rn(t[1], t[1]), t[1],
-                                   fmaf(__fmul_rn(t[2], t[2]), t[2],
-                                        __fmul_rn(__fmul_rn(t[3], t[3]), t[3]))));
+        const float yb = fmaf(t2[0], t[0], fmaf(t2[1], t[1],
+                              fmaf(t2[2], t[2], __fmul_rn(t2[3], t[3]))));
         const float y = yb - comp;
         const float s = st + y;
         comp = (s - st) - y;
@@ -212,11 +283,24 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksDensity)
 //   15 own predicted displacement along the gravity axis / h
 // RAW: FP32 features to feat[p][16]; otherwise the network's input row
 // bf16((f - mean) * inv_std) (norm = mean[16], inv_std[16]) to xbf[p][16].
+// It gathers the 32-byte particle records; in a block with a tile the slots of
+// the tile's records are laid out in shared memory for that.
 template <bool RAW>
-__global__ void __launch_bounds__(kBlock, kMinBlocksFeatures)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocksFeatures)
     k_features(const DevParams P, const NbrView V, const PassArgs a, float* __restrict__ feat,
                __nv_bfloat16* __restrict__ xbf, const float* __restrict__ norm, int limit) {
+  __shared__ int s_slot[kTileCap];
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const TileInfo* info = V.tiles + blockIdx.x;
+  const int total = __ldg(&info->total);
+  if (total >= 0) {
+    for (int r = 0; r < 9; ++r) {
+      const int s = __ldg(&info->s[r]), o = __ldg(&info->o[r]),
+                len = (r < 8 ? __ldg(&info->o[r + 1]) : total) - o;
+      for (int t = threadIdx.x; t < len; t += kTileSlots) s_slot[o + t] = s + t;
+    }
+    __syncthreads();
+  }
   double err = 0.0;
   if (p < P.n) {
     float4 xp, dp;
@@ -229,12 +313,31 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksFeatures)
     float st = 0.0f, comp = 0.0f;
     float sgx = 0.f, sgy = 0.f, sgz = 0.f, sC = 0.f;
     float ox = 0.f, oy = 0.f, oz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f, rmin2 = P.h2;
-    int cnt = 0;
-    for_each_batch_pd<kNbrBatch>(V, a.pd, p, [&](const float4 (&xq)[kNbrBatch],
-                                                 const float4 (&dq)[kNbrBatch], int nvalid) {
+    const int cnt = (int)__ldg(V.ncount + p);
+    uint4 blk = cnt > 0 ? nbr_block(V, p, 0) : make_uint4(0u, 0u, 0u, 0u);
+    for (int j0 = 0; j0 < cnt; j0 += 4) {
+      const int nvalid = cnt - j0;
+      int q[4];
+      if (total >= 0) {
+        // the low half of a block, then the high half, eight entries in all
+        const uint32_t w0 = (j0 & 4) ? blk.z : blk.x, w1 = (j0 & 4) ? blk.w : blk.y;
+        const uint32_t o[4] = {w0 & 0xffffu, w0 >> 16, w1 & 0xffffu, w1 >> 16};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = s_slot[o[u] >> 4];
+        if ((j0 & 4) && j0 + 4 < cnt) blk = nbr_block(V, p, (j0 >> 3) + 1);
+      } else {
+        q[0] = (int)blk.x;
+        q[1] = (int)blk.y;
+        q[2] = (int)blk.z;
+        q[3] = (int)blk.w;
+        if (j0 + 4 < cnt) blk = nbr_block(V, p, (j0 >> 2) + 1);
+      }
+      float4 xq[4], dq[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) ld_pd(a.pd, q[u], xq[u], dq[u]);
       float yb = 0.0f;
 #pragma unroll
-      for (int u = 0; u < kNbrBatch; ++u) {
+      for (int u = 0; u < 4; ++u) {
         if (u < nvalid) {
           const Pair g = pair_geom(xp, dp, xq[u], dq[u]);
           const float t = fmaxf(P.h2 - g.r2, 0.0f);
@@ -254,14 +357,13 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksFeatures)
           uy += dq[u].y;
           uz += dq[u].z;
           rmin2 = fminf(rmin2, g.r2);
-          ++cnt;
         }
       }
       const float y = yb - comp;
       const float s = st + y;
       comp = (s - st) - y;
       st = s;
-    });
+    }
     // sum_q (d_q - d_p) from sum_q d_q
     ux = fmaf(-(float)cnt, dp.x, ux);
     uy = fmaf(-(float)cnt, dp.y, uy);
@@ -334,11 +436,12 @@ __global__ void k_accum_lambda(const uint4* __restrict__ rec, float s, float* __
 }
 
 template <int MODE, int SCORR_N, bool SDF>
-__global__ void __launch_bounds__(kBlock, kMinBlocksPosition)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
     k_position(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const uint4 rp = ld_nr(a.nr, p);
+  SPHPC_PASS_HEAD(1, a.nr, nullptr);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  SPHPC_PASS_READY();
+  if (!own) return;
   const float lp = nr_w(rp);
   float4 xp, dp;  // own particle record, loaded ahead of the neighbour loop
   if (MODE == 0) ld_pd(a.pd, p, xp, dp);
@@ -347,33 +450,38 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPosition)
   // and 2^-2k multiply them once afterwards.  Every term carries d, so the batch's
   // padding slots (q = p, d = 0) add nothing and are not masked.
   float ax = 0.f, ay = 0.f, az = 0.f;
-  for_each_neighbor_nr<kNbrBatch, true>(V, a.nr, p, [&](int, const uint4 rq) {
-    const float fx = (float)(int)(rp.x - rq.x);
-    const float fy = (float)(int)(rp.y - rq.y);
-    const float fz = (float)(int)(rp.z - rq.z);
-    // in fixed-point units: c_f = s (h_f - r_f)^2 / r_f = 2^k c
-    float r2c, rinv;
-    floored_r_fx(P, norm2(fx, fy, fz), r2c, rinv);
-    const float hm = fx_hm(P, r2c, rinv);
-    float s = lp + nr_w(rq);
-    if (SCORR_N != 0) {
-      // W(r) / W(dq) = u^3 with u = (h^2 - r^2) / (h^2 - dq^2), u <= 1.05
-      const float u = fmaxf(fmaf(-P.scorr_u_fx, r2c, P.scorr_uh2), 0.0f);
-      if (SCORR_N == 4) {
-        const float u2 = u * u;
-        const float u4 = u2 * u2;
-        s = fmaf(-P.scorr_k, u4 * u4 * u4, s);
-      } else {
-        const float ratio = u * u * u;
-        float sc = -P.scorr_k;
-        for (int e = 0; e < P.scorr_n; ++e) sc = __fmul_rn(sc, ratio);
-        s = __fadd_rn(s, sc);
+  visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk, [&](const Batch<1>& q, int) {
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {
+      const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
+      // in fixed-point units: c_f = s (h_f - r_f)^2 / r_f = 2^k c
+      const uint64_t r2c = max2(norm2_2(d), P.rmin2_fx);
+      const uint64_t rinv = rsqrt2(r2c);
+      const uint64_t hm = h_minus_r(P, r2c, rinv);
+      uint64_t s = f2_pack(lp + nr_w(q.r[u]), lp + nr_w(q.r[u + 1]));
+      if (SCORR_N != 0) {
+        // W(r) / W(dq) = w^3 with w = (h^2 - r^2) / (h^2 - dq^2), w <= 1.05
+        const uint64_t w =
+            max2(f2_fma(f2_dup(-P.scorr_u_fx), r2c, f2_dup(P.scorr_uh2)), 0.0f);
+        if (SCORR_N == 4) {
+          const uint64_t w2 = f2_mul(w, w);
+          const uint64_t w4 = f2_mul(w2, w2);
+          s = f2_fma(f2_dup(-P.scorr_k), f2_mul(f2_mul(w4, w4), w4), s);
+        } else {
+          const uint64_t ratio = f2_mul(f2_mul(w, w), w);
+          uint64_t sc = f2_dup(-P.scorr_k);
+          for (int e = 0; e < P.scorr_n; ++e) sc = f2_mul(sc, ratio);
+          s = f2_add(s, sc);
+        }
       }
+      const uint64_t c = f2_mul(f2_mul(f2_mul(s, hm), hm), rinv);
+      ax = fmaf(f2_lo(c), f2_lo(d.x), ax);
+      ay = fmaf(f2_lo(c), f2_lo(d.y), ay);
+      az = fmaf(f2_lo(c), f2_lo(d.z), az);
+      ax = fmaf(f2_hi(c), f2_hi(d.x), ax);
+      ay = fmaf(f2_hi(c), f2_hi(d.y), ay);
+      az = fmaf(f2_hi(c), f2_hi(d.z), az);
     }
-    const float c = __fmul_rn(__fmul_rn(__fmul_rn(s, hm), hm), rinv);
-    ax = fmaf(c, fx, ax);
-    ay = fmaf(c, fy, ay);
-    az = fmaf(c, fz, az);
   });
   const float s = a.stiffness * P.inv_rho0 * (P.DWn_m * P.fx_inv2);
   const float dpx = ax * s, dpy = ay * s, dpz = az * s;
@@ -428,40 +536,37 @@ __global__ void __launch_bounds__(kBlock) k_apply_dp(const DevParams P, const Pa
                               __double2float_rn(__dsub_rn(zs, (double)xp.z)), dp.w);
 }
 
-__global__ void __launch_bounds__(kBlock) k_pack_nv(int n, const uint4* __restrict__ nr,
-                                                    const float4* __restrict__ e,
-                                                    NV* __restrict__ nv) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) st_nv(nv, p, ld_nr(nr, p), __ldg(e + p));
-}
-
-__global__ void __launch_bounds__(kBlock, kMinBlocksColor)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
     k_color(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const uint4 rp = ld_nr(a.nr, p);
+  SPHPC_PASS_HEAD(1, a.nr, nullptr);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  SPHPC_PASS_READY();
+  if (!own) return;
   // sums of (h^2 - r^2)^2 r / (r rho_q) d, d in fixed-point units; the
   // poly6-gradient norm, m, h and 2^-k multiply them once (every term carries
   // d, so the padding slots add nothing)
   float cx = 0.f, cy = 0.f, cz = 0.f;
-  for_each_neighbor_nr<kNbrBatch, true>(V, a.nr, p, [&](int, const uint4 rq) {
-    const float fx = (float)(int)(rp.x - rq.x);
-    const float fy = (float)(int)(rp.y - rq.y);
-    const float fz = (float)(int)(rp.z - rq.z);
-    // r and 1/r in fixed-point units (their product is unit-free)
-    float r2c, rinv;
-    floored_r_fx(P, norm2(fx, fy, fz), r2c, rinv);
-    const float t = fmaxf(fmaf(-P.fx_inv2, r2c, P.h2), 0.0f);
-    const float c = __fmul_rn(__fmul_rn(__fmul_rn(t, t), fx_r(r2c, rinv)),
-                              __fmul_rn(rinv, rcp_fast(nr_w(rq))));
-    cx = fmaf(c, fx, cx);
-    cy = fmaf(c, fy, cy);
-    cz = fmaf(c, fz, cz);
+  visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk, [&](const Batch<1>& q, int) {
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {
+      const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
+      // r and 1/r in fixed-point units (their product is unit-free)
+      const uint64_t r2c = max2(norm2_2(d), P.rmin2_fx);
+      const uint64_t rinv = rsqrt2(r2c);
+      const uint64_t t = max2(f2_fma(f2_dup(-P.fx_inv2), r2c, f2_dup(P.h2)), 0.0f);
+      const uint64_t irho = f2_pack(rcp_fast(nr_w(q.r[u])), rcp_fast(nr_w(q.r[u + 1])));
+      const uint64_t c =
+          f2_mul(f2_mul(f2_mul(t, t), f2_mul(r2c, rinv)), f2_mul(rinv, irho));
+      cx = fmaf(f2_lo(c), f2_lo(d.x), cx);
+      cy = fmaf(f2_lo(c), f2_lo(d.y), cy);
+      cz = fmaf(f2_lo(c), f2_lo(d.z), cz);
+      cx = fmaf(f2_hi(c), f2_hi(d.x), cx);
+      cy = fmaf(f2_hi(c), f2_hi(d.y), cy);
+      cz = fmaf(f2_hi(c), f2_hi(d.z), cz);
+    }
   });
   const float s = P.h * (P.DWPn * P.m * P.fx_inv);
-  const float4 col = make_float4(s * cx, s * cy, s * cz, 0.0f);
-  a.color[p] = col;
-  if (a.nv_out) st_nv(a.nv_out, p, rp, col);
+  a.color[p] = make_float4(s * cx, s * cy, s * cz, 0.0f);
 }
 
 // Akinci cohesion spline (particles.c:54-65) without its norm: with
@@ -474,13 +579,13 @@ __device__ __forceinline__ float cohesion_unnormed(const DevParams& P, float r, 
   return r > P.h ? 0.0f : c;
 }
 
-__global__ void __launch_bounds__(kBlock, kMinBlocksTension)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks2)
     k_tension(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  uint4 recp;
-  float4 cp;
-  ld_nv(a.nv, p, recp, cp);
+  SPHPC_PASS_HEAD(2, a.nr, a.color);
+  const uint4 recp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  const float4 cp = own ? __ldg(a.color + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+  SPHPC_PASS_READY();
+  if (!own) return;
   const float rp = nr_w(recp);
   const float kcoh = -20.0f * P.gamma * P.m * P.m;
   const float kcur = -P.gamma * P.m;
@@ -494,7 +599,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksTension)
   // kcur (c_p - c_q) = kcur c_p - kcur c_q
   const float kpx = kcur * cp.x, kpy = kcur * cp.y, kpz = kcur * cp.z;
   float fx = 0.f, fy = 0.f, fz = 0.f;
-  for_each_neighbor_nv<kNbrBatch, true>(V, a.nv, p, [&](int, const uint4 rq, const float4 cq) {
+  visit<2>(V, tiled, tile, a.nr, a.color, p, cnt, blk, [&](const Batch<2>& q, int) {
+#pragma unroll
+   for (int u = 0; u < 4; ++u) {
+    const uint4 rq = q.r[u];
+    const float4 cq = q.e[u];
     const float dx = (float)(int)(recp.x - rq.x);
     const float dy = (float)(int)(recp.y - rq.y);
     const float dz = (float)(int)(recp.z - rq.z);
@@ -506,6 +615,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksTension)
     fx = fmaf(K, fmaf(coh, dx, fmaf(-kcur, cq.x, kpx)), fx);
     fy = fmaf(K, fmaf(coh, dy, fmaf(-kcur, cq.y, kpy)), fy);
     fz = fmaf(K, fmaf(coh, dz, fmaf(-kcur, cq.z, kpz)), fz);
+   }
   });
   float4 v = a.vel[p];
   const float s = P.dt / rp;
@@ -513,20 +623,23 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksTension)
   v.y = fmaf(s, fy, v.y);
   v.z = fmaf(s, fz, v.z);
   a.vel[p] = v;
-  if (a.nv_out) st_nv(a.nv_out, p, recp, v);
 }
 
-__global__ void __launch_bounds__(kBlock, kMinBlocksXsph)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks2)
     k_xsph(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  uint4 rp;
-  float4 vp;
-  ld_nv(a.nv, p, rp, vp);
+  SPHPC_PASS_HEAD(2, a.nr, a.vel);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  const float4 vp = own ? __ldg(a.vel + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+  SPHPC_PASS_READY();
+  if (!own) return;
   // sums of (v_q - v_p) t^3 / rho_q; the poly6 norm, m and c multiply them
   // once (the padding slots' v_q - v_p is 0)
   float sx = 0.f, sy = 0.f, sz = 0.f;
-  for_each_neighbor_nv<kNbrBatch, true>(V, a.nv, p, [&](int, const uint4 rq, const float4 vq) {
+  visit<2>(V, tiled, tile, a.nr, a.vel, p, cnt, blk, [&](const Batch<2>& q, int) {
+#pragma unroll
+   for (int u = 0; u < 4; ++u) {
+    const uint4 rq = q.r[u];
+    const float4 vq = q.e[u];
     const Pair g = pair_nr(P, rp, rq);
     // particles.c:439 evaluates x^2 + y^2 * z^2 (kept unless xsph_exact)
     const float rr =
@@ -537,11 +650,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksXsph)
     sx = fmaf(vq.x - vp.x, w, sx);
     sy = fmaf(vq.y - vp.y, w, sy);
     sz = fmaf(vq.z - vp.z, w, sz);
+   }
   });
   const float cw = P.c_xsph * P.Wn_m;
   const float4 vn = make_float4(fmaf(cw, sx, vp.x), fmaf(cw, sy, vp.y), fmaf(cw, sz, vp.z), 0.0f);
   a.vel_out[p] = vn;
-  if (a.nv_out) st_nv(a.nv_out, p, rp, vn);
   if (a.write_pos) {
     float4 xp, dp;
     ld_pd(a.pd, p, xp, dp);
@@ -555,18 +668,22 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksXsph)
 
 // With nr_out, also the records {X, |omega|} the confinement pass gathers
 // (one 16-byte load per neighbour instead of a record and omega[q]).
-__global__ void __launch_bounds__(kBlock, kMinBlocksVorticity)
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks2)
     k_vorticity(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  uint4 rp;
-  float4 vp;
-  ld_nv(a.nv, p, rp, vp);
+  SPHPC_PASS_HEAD(2, a.nr, a.vel);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  const float4 vp = own ? __ldg(a.vel + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+  SPHPC_PASS_READY();
+  if (!own) return;
   // sums of (v_q - v_p) x c d with c = (h - r)^2 / r and d in fixed-point
   // units (r too); the spiky norm and 2^-2k multiply them once (the padding slots'
   // v_q - v_p and d are 0)
   float wx = 0.f, wy = 0.f, wz = 0.f;
-  for_each_neighbor_nv<kNbrBatch, true>(V, a.nv, p, [&](int, const uint4 rq, const float4 vq) {
+  visit<2>(V, tiled, tile, a.nr, a.vel, p, cnt, blk, [&](const Batch<2>& q, int) {
+#pragma unroll
+   for (int u = 0; u < 4; ++u) {
+    const uint4 rq = q.r[u];
+    const float4 vq = q.e[u];
     const float dx = (float)(int)(rp.x - rq.x);
     const float dy = (float)(int)(rp.y - rq.y);
     const float dz = (float)(int)(rp.z - rq.z);
@@ -579,6 +696,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksVorticity)
     wx = __fadd_rn(wx, fmaf(uy, gz, -__fmul_rn(uz, gy)));
     wy = __fadd_rn(wy, fmaf(uz, gx, -__fmul_rn(ux, gz)));
     wz = __fadd_rn(wz, fmaf(ux, gy, -__fmul_rn(uy, gx)));
+   }
   });
   const float sw = P.DWn * P.fx_inv2;
   wx *= sw;
@@ -589,29 +707,32 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksVorticity)
   if (a.nr_out) a.nr_out[p] = make_uint4(rp.x, rp.y, rp.z, __float_as_uint(wm));
 }
 
-// OW: a.nr carries |omega| as its payload (the vorticity pass's records);
-// otherwise |omega_q| comes from omega[q].w.
-template <bool OW>
-__global__ void __launch_bounds__(kBlock, kMinBlocksConfinement)
+// a.nr carries |omega| as its payload (the vorticity pass's records).
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
     k_confinement(const DevParams P, const NbrView V, const PassArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const uint4 rp = ld_nr(a.nr, p);
+  SPHPC_PASS_HEAD(1, a.nr, nullptr);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  SPHPC_PASS_READY();
+  if (!own) return;
   // sums of |omega_q| (h - r)^2 / r d, d and r in fixed-point units; the
   // spiky norm and 2^-2k multiply them once (the padding slots' d is 0)
   float ex = 0.f, ey = 0.f, ez = 0.f;
-  for_each_neighbor_nr<kNbrBatch, true>(V, a.nr, p, [&](int q, const uint4 rq) {
-    const float dx = (float)(int)(rp.x - rq.x);
-    const float dy = (float)(int)(rp.y - rq.y);
-    const float dz = (float)(int)(rp.z - rq.z);
-    float r2c, rinv;
-    floored_r_fx(P, norm2(dx, dy, dz), r2c, rinv);
-    const float hm = fx_hm(P, r2c, rinv);
-    const float wq = OW ? nr_w(rq) : __ldg(a.omega + q).w;
-    const float c = __fmul_rn(__fmul_rn(__fmul_rn(hm, hm), rinv), wq);
-    ex = fmaf(c, dx, ex);
-    ey = fmaf(c, dy, ey);
-    ez = fmaf(c, dz, ez);
+  visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk, [&](const Batch<1>& q, int) {
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {
+      const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
+      const uint64_t r2c = max2(norm2_2(d), P.rmin2_fx);
+      const uint64_t rinv = rsqrt2(r2c);
+      const uint64_t hm = h_minus_r(P, r2c, rinv);
+      const uint64_t g = f2_mul(f2_mul(hm, hm), rinv);
+      const float ca = __fmul_rn(f2_lo(g), nr_w(q.r[u])), cb = __fmul_rn(f2_hi(g), nr_w(q.r[u + 1]));
+      ex = fmaf(ca, f2_lo(d.x), ex);
+      ey = fmaf(ca, f2_lo(d.y), ey);
+      ez = fmaf(ca, f2_lo(d.z), ez);
+      ex = fmaf(cb, f2_hi(d.x), ex);
+      ey = fmaf(cb, f2_hi(d.y), ey);
+      ez = fmaf(cb, f2_hi(d.z), ez);
+    }
   });
   const float se = P.DWn * P.fx_inv2;
   ex *= se;
@@ -633,7 +754,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksConfinement)
           make_float4(__double2float_rn(xstar_d(xp.x, dp.x)),
                       __double2float_rn(xstar_d(xp.y, dp.y)),
                       __double2float_rn(xstar_d(xp.z, dp.z)), 0.0f),
-          make_float4(0.f, 0.f, 0.f, OW ? 0.0f : nr_w(rp)));
+          make_float4(0.f, 0.f, 0.f, 0.0f));
   }
 }
 
@@ -707,15 +828,15 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // 16-byte records from the particle records: canonical x* = x + d and the
-// payload src[p] (d.w without src).
+// payload src[p * stride] (d.w without src).
 __global__ void __launch_bounds__(kBlock)
     k_make_nr(const DevParams P, const PD* __restrict__ pd, const float* __restrict__ src,
-              uint4* __restrict__ nr) {
+              int stride, uint4* __restrict__ nr) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P.n) return;
   const float4 x = pd[p].x, d = pd[p].d;
   nr[p] = make_nr(P, xstar_d(x.x, d.x), xstar_d(x.y, d.y), xstar_d(x.z, d.z),
-                  src ? src[p] : d.w);
+                  src ? src[(size_t)p * stride] : d.w);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -732,28 +853,32 @@ __global__ void __launch_bounds__(kBlock)
 
 }  // namespace
 
+// Launch of a neighbour pass with the tiles of NARR arrays.
+#define SPHPC_COMMA ,
+#define SPHPC_PASS(NARR, kernel) \
+  kernel<<<grid_for(P.n, kTileSlots), kTileSlots, NARR * kTileCap * 16, st>>>(P, V, a)
+
 void launch_density_lambda(const DevParams& P, const NbrView& V, const PassArgs& a, int mode,
                            bool residual, cudaStream_t st) {
-  const int g = grid_for(P.n);
   if (mode == 0) {
-    if (residual) k_density_lambda<0, true><<<g, kBlock, 0, st>>>(P, V, a);
-    else k_density_lambda<0, false><<<g, kBlock, 0, st>>>(P, V, a);
+    if (residual) SPHPC_PASS(1, k_density_lambda<0 SPHPC_COMMA true>);
+    else SPHPC_PASS(1, k_density_lambda<0 SPHPC_COMMA false>);
   } else if (mode == 1) {
-    if (residual) k_density_lambda<1, true><<<g, kBlock, 0, st>>>(P, V, a);
-    else k_density_lambda<1, false><<<g, kBlock, 0, st>>>(P, V, a);
+    if (residual) SPHPC_PASS(1, k_density_lambda<1 SPHPC_COMMA true>);
+    else SPHPC_PASS(1, k_density_lambda<1 SPHPC_COMMA false>);
   } else {
-    k_density_lambda<2, false><<<g, kBlock, 0, st>>>(P, V, a);
+    SPHPC_PASS(1, k_density_lambda<2 SPHPC_COMMA false>);
   }
 }
 
 void launch_features(const DevParams& P, const NbrView& V, const PassArgs& a, float* feat,
                      int limit, cudaStream_t st) {
-  k_features<true><<<grid_for(P.n), kBlock, 0, st>>>(P, V, a, feat, nullptr, nullptr, limit);
+  k_features<true><<<grid_for(P.n, kTileSlots), kTileSlots, 0, st>>>(P, V, a, feat, nullptr, nullptr, limit);
 }
 
 void launch_features_bf16(const DevParams& P, const NbrView& V, const PassArgs& a,
                           __nv_bfloat16* xbf, const float* norm, cudaStream_t st) {
-  k_features<false><<<grid_for(P.n), kBlock, 0, st>>>(P, V, a, nullptr, xbf, norm, P.n);
+  k_features<false><<<grid_for(P.n, kTileSlots), kTileSlots, 0, st>>>(P, V, a, nullptr, xbf, norm, P.n);
 }
 
 void launch_accum_lambda(const uint4* rec, float s, float* target, int limit, cudaStream_t st) {
@@ -762,10 +887,10 @@ void launch_accum_lambda(const uint4* rec, float s, float* target, int limit, cu
 
 void launch_position(const DevParams& P, const NbrView& V, const PassArgs& a, int mode,
                      cudaStream_t st) {
-  const int g = grid_for(P.n);
   const int sn = P.scorr_k != 0.0f ? (P.scorr_n == 4 ? 4 : -1) : 0;
   const bool sdf = P.has_sdf != 0;
-#define SPHPC_POS(M, N, S) k_position<M, N, S><<<g, kBlock, 0, st>>>(P, V, a)
+#define SPHPC_POS(M, N, S) \
+  SPHPC_PASS(1, k_position<M SPHPC_COMMA N SPHPC_COMMA S>)
   if (mode == 0) {
     if (sn == 0) { if (sdf) SPHPC_POS(0, 0, true); else SPHPC_POS(0, 0, false); }
     else if (sn == 4) { if (sdf) SPHPC_POS(0, 4, true); else SPHPC_POS(0, 4, false); }
@@ -783,25 +908,21 @@ void launch_apply_dp(const DevParams& P, const PassArgs& a, cudaStream_t st) {
   else k_apply_dp<false><<<grid_for(P.n), kBlock, 0, st>>>(P, a);
 }
 
-void launch_pack_nv(int n, const uint4* nr, const float4* e, NV* nv, cudaStream_t st) {
-  if (n > 0) k_pack_nv<<<grid_for(n), kBlock, 0, st>>>(n, nr, e, nv);
-}
 void launch_color(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st) {
-  k_color<<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
+  SPHPC_PASS(1, k_color);
 }
 void launch_tension(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st) {
-  k_tension<<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
+  SPHPC_PASS(2, k_tension);
 }
 void launch_xsph(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st) {
-  k_xsph<<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
+  SPHPC_PASS(2, k_xsph);
 }
 void launch_vorticity(const DevParams& P, const NbrView& V, const PassArgs& a, cudaStream_t st) {
-  k_vorticity<<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
+  SPHPC_PASS(2, k_vorticity);
 }
-void launch_confinement(const DevParams& P, const NbrView& V, const PassArgs& a, bool omega_in_nr,
+void launch_confinement(const DevParams& P, const NbrView& V, const PassArgs& a,
                         cudaStream_t st) {
-  if (omega_in_nr) k_confinement<true><<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
-  else k_confinement<false><<<grid_for(P.n), kBlock, 0, st>>>(P, V, a);
+  SPHPC_PASS(1, k_confinement);
 }
 void launch_gravity(const DevParams& P, float4* vel, cudaStream_t st) {
   k_gravity<<<grid_for(P.n), kBlock, 0, st>>>(P, vel);
@@ -820,8 +941,8 @@ void launch_pack_w(const DevParams& P, PD* pd, uint4* nr, const float* src, cuda
   k_pack_w<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, nr, src);
 }
 void launch_make_nr(const DevParams& P, const PD* pd, const float* src, uint4* nr,
-                    cudaStream_t st) {
-  k_make_nr<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, src, nr);
+                    cudaStream_t st, int stride) {
+  k_make_nr<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, src, stride, nr);
 }
 void launch_collisions_double(const DevParams& P, double* x, double* y, double* z, int n,
                               cudaStream_t st) {

@@ -92,7 +92,7 @@ class DeviceSim {
   uint32_t* keys_sorted = nullptr;  // view into keys_by_id or sort.keys_alt
   uint32_t *cellp = nullptr, *nbr = nullptr, *cstart = nullptr;
   float4* xsa = nullptr;
-  NV *nv_a = nullptr, *nv_b = nullptr;  // combined records of the post passes
+  TileInfo* tiles = nullptr;  // of the current lists
   uint8_t* ncount = nullptr;
   uint4* gaps = nullptr;
   uint32_t* small = nullptr;  // [0] gap count, [1] explicit count, [2] error bits
@@ -168,7 +168,7 @@ class DeviceSim {
     dfree(color); dfree(omega); dfree(dp); dfree(rho); dfree(lam);
     dfree(color_alt); dfree(omega_alt); dfree(dp_alt); dfree(rho_alt); dfree(lam_alt);
     dfree(ids); dfree(ids_spare); dfree(keys_by_id); dfree(loc_by_id); dfree(cellp);
-    dfree(nbr); dfree(xsa); dfree(nv_a); dfree(nv_b);
+    dfree(nbr); dfree(xsa); dfree(tiles);
     dfree(cstart); dfree(ncount); dfree(gaps); dfree(small);
     dfree(resid); dfree(sort.keys_alt); dfree(sort.vals_alt); dfree(sort_aux); dfree(stage);
     mlp_release(mlp);
@@ -190,16 +190,17 @@ class DeviceSim {
     cap = cap_ > n_ ? cap_ : n_;
     const int c = cap;
     SPHPC_RC(dalloc(&pd, c)); SPHPC_RC(dalloc(&pd_alt, c));
-    SPHPC_RC(dalloc(&nr, c)); SPHPC_RC(dalloc(&nr_alt, c));
-    SPHPC_RC(dalloc(&vel, c)); SPHPC_RC(dalloc(&vel_alt, c));
-    SPHPC_RC(dalloc(&color, c)); SPHPC_RC(dalloc(&omega, c)); SPHPC_RC(dalloc(&dp, c));
+    // arrays that tiles are copied from: ranges end on an even slot
+    SPHPC_RC(dalloc(&nr, (size_t)c + 2)); SPHPC_RC(dalloc(&nr_alt, (size_t)c + 2));
+    SPHPC_RC(dalloc(&vel, (size_t)c + 2)); SPHPC_RC(dalloc(&vel_alt, (size_t)c + 2));
+    SPHPC_RC(dalloc(&color, (size_t)c + 2)); SPHPC_RC(dalloc(&omega, c)); SPHPC_RC(dalloc(&dp, c));
     SPHPC_RC(dalloc(&rho, c)); SPHPC_RC(dalloc(&lam, c));
     SPHPC_RC(dalloc(&ids, c)); SPHPC_RC(dalloc(&ids_spare, c));
     SPHPC_RC(dalloc(&keys_by_id, c)); SPHPC_RC(dalloc(&loc_by_id, c));
     SPHPC_RC(dalloc(&cellp, c)); SPHPC_RC(dalloc(&ncount, c));
     SPHPC_RC(dalloc(&nbr, (size_t)kMaxNeighbors * c));
-    SPHPC_RC(dalloc(&xsa, (size_t)c + 2));  // pair blocks: 32 bytes per slot pair
-    SPHPC_RC(dalloc(&nv_a, c)); SPHPC_RC(dalloc(&nv_b, c));
+    SPHPC_RC(dalloc(&xsa, (size_t)c + 4));  // pair blocks; the build reads four slots at a time
+    SPHPC_RC(dalloc(&tiles, (size_t)grid_for(c, kTileSlots)));
     SPHPC_CK(cudaMemsetAsync(ncount, 0, c, stream));
     SPHPC_RC(dalloc(&small, 8));
     SPHPC_RC(dalloc(&resid, 16));
@@ -223,7 +224,7 @@ class DeviceSim {
   }
 
   int ensure_full_alts() {
-    if (!color_alt) SPHPC_RC(dalloc(&color_alt, cap));
+    if (!color_alt) SPHPC_RC(dalloc(&color_alt, (size_t)cap + 2));
     if (!omega_alt) SPHPC_RC(dalloc(&omega_alt, cap));
     if (!dp_alt) SPHPC_RC(dalloc(&dp_alt, cap));
     if (!rho_alt) SPHPC_RC(dalloc(&rho_alt, cap));
@@ -293,6 +294,8 @@ class DeviceSim {
     v.nbr = nbr;
     v.ncount = ncount;
     v.cstart = cstart;
+    v.tiles = tiles;
+    v.err = small + 2;
     v.n = n;
     v.nx = nx; v.ny = ny; v.nz = nz;
     v.nxny = (uint32_t)nx * (uint32_t)ny;
@@ -391,7 +394,7 @@ class DeviceSim {
   int run_step(const DevParams& P, const Params& prm);
 
   int ensure_carry_buffers() {
-    if (!nr_w) SPHPC_RC(dalloc(&nr_w, cap));
+    if (!nr_w) SPHPC_RC(dalloc(&nr_w, (size_t)cap + 2));
     if (!lam_acc) {
       SPHPC_RC(dalloc(&lam_acc, cap));
       have_carry = false;
@@ -400,7 +403,7 @@ class DeviceSim {
   }
 
   int ensure_warm_buffers() {
-    if (!nr_w) SPHPC_RC(dalloc(&nr_w, cap));
+    if (!nr_w) SPHPC_RC(dalloc(&nr_w, (size_t)cap + 2));
     if (mlp.feat_cap < cap) {
       if (mlp.feat) cudaFree(mlp.feat);
       mlp.feat = nullptr;
@@ -443,9 +446,11 @@ DevParams DeviceSim::params(const Params& prm, const AABB* b, const Obstacle* ob
     if (sphpc_neighbor_pretest_fp32_safe((double)nmax * h, h)) {
       P.bld_h2lo = (float)(h * h) * (1.0f - 1.0f / 1024.0f);
       P.bld_h2hi = (float)(h * h) * (1.0f + 1.0f / 1024.0f);
+      P.bld_band = (float)(h * h) * (1.0f / 1024.0f);
     } else {
       P.bld_h2lo = -1.0f;
       P.bld_h2hi = INFINITY;
+      P.bld_band = INFINITY;
     }
   }
   P.h = (float)h;
@@ -593,7 +598,7 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
   }
   {
     Scope sc(this, "build_neighbors");
-    launch_build_neighbors(P, view(), pd, xsa, cellp, nbr, ncount, stream);
+    launch_build_neighbors(P, view(), pd, xsa, cellp, nbr, ncount, tiles, stream);
     launches += 1;
   }
   SPHPC_CK(cudaGetLastError());
@@ -816,28 +821,17 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
   a.pd_out = pd_alt;
   a.nr = nr;
   a.nr_out = nullptr;
-  // each pass that gathers the neighbours' velocities (or colours) with their
-  // records reads them from combined 32-byte records {nr, v} written by the
-  // pass before it
   if (solver.surface_tension) {
     Scope sc(this, "surface_tension");
     a.color = color;
-    a.nv_out = nv_a;
-    launch_color(P, V, a, stream);
     a.vel = vel;
-    a.nv = nv_a;
-    a.nv_out = nv_b;
+    launch_color(P, V, a, stream);
     launch_tension(P, V, a, stream);
     launches += 2;
   }
   {
     Scope sc(this, "xsph");
-    if (!solver.surface_tension) {
-      launch_pack_nv(n, nr, vel, nv_b, stream);
-      launches += 1;
-    }
-    a.nv = nv_b;
-    a.nv_out = solver.vorticity ? nv_a : nullptr;
+    a.vel = vel;
     a.vel_out = vel_alt;
     a.write_pos = solver.vorticity ? 0 : 1;
     launch_xsph(P, V, a, stream);
@@ -847,8 +841,6 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
     Scope sc(this, "vorticity");
     // the vorticity pass also writes the records {X, |omega|} (into nr_alt)
     // that the confinement pass gathers
-    a.nv = nv_a;
-    a.nv_out = nullptr;
     a.vel = vel_alt;
     a.omega = omega;
     a.nr_out = nr_alt;
@@ -857,7 +849,7 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
     a.nr = nr_alt;
     a.nr_out = nullptr;
     a.write_pos = 1;
-    launch_confinement(P, V, a, true, stream);
+    launch_confinement(P, V, a, stream);
     launches += 2;
   }
   std::swap(vel, vel_alt);
@@ -1473,10 +1465,7 @@ int ComputeSurfaceTension(struct Particles* particles, const struct Params* para
   a.nr = s->nr;
   a.color = s->color;
   a.vel = s->vel;
-  a.nv_out = s->nv_a;
   launch_color(P, s->view(), a, s->stream);
-  a.nv = s->nv_a;
-  a.nv_out = nullptr;
   launch_tension(P, s->view(), a, s->stream);
   SPHPC_LAUNCH_DONE();
 }
@@ -1489,11 +1478,9 @@ int ApplyViscosity(struct Particles* particles, const struct Params* params,
   const DevParams P = s->params(*params, nullptr, nullptr);
   launch_pack_w(P, s->pd, nullptr, s->rho, s->stream);
   launch_make_nr(P, s->pd, s->rho, s->nr, s->stream);
-  launch_pack_nv(s->n, s->nr, s->vel, s->nv_a, s->stream);
   PassArgs a{};
   a.pd = s->pd;
   a.nr = s->nr;
-  a.nv = s->nv_a;
   a.vel = s->vel;
   a.vel_out = s->vel_alt;
   launch_xsph(P, s->view(), a, s->stream);
@@ -1508,11 +1495,9 @@ int ComputeVorticity(struct Particles* particles, const struct Params* params,
   SPHPC_NEED_NBR();
   const DevParams P = s->params(*params, nullptr, nullptr);
   launch_make_nr(P, s->pd, nullptr, s->nr, s->stream);
-  launch_pack_nv(s->n, s->nr, s->vel, s->nv_a, s->stream);
   PassArgs a{};
   a.pd = s->pd;
   a.nr = s->nr;
-  a.nv = s->nv_a;
   a.vel = s->vel;
   a.omega = s->omega;
   launch_vorticity(P, s->view(), a, s->stream);
@@ -1525,13 +1510,14 @@ int ApplyVorticityConfinement(struct Particles* particles, const struct Params* 
   SPHPC_STAGE_BEGIN(particles, params);
   SPHPC_NEED_NBR();
   const DevParams P = s->params(*params, nullptr, nullptr);
-  launch_make_nr(P, s->pd, nullptr, s->nr, s->stream);
+  // the records' payload is |omega|, the fourth component of omega
+  launch_make_nr(P, s->pd, reinterpret_cast<const float*>(s->omega) + 3, s->nr, s->stream, 4);
   PassArgs a{};
   a.pd = s->pd;
   a.nr = s->nr;
   a.vel = s->vel;
   a.omega = s->omega;
-  launch_confinement(P, s->view(), a, false, s->stream);
+  launch_confinement(P, s->view(), a, s->stream);
   SPHPC_LAUNCH_DONE();
 }
 

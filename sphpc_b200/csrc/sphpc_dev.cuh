@@ -20,11 +20,14 @@
 //   ids[n]   u32     original particle index of each slot
 //   cellp[n] u32     packed grid cell (cx | cy<<bx | cz<<(bx+by)) of x* at
 //                    neighbour-build time
-//   nbr4[15][n] uint4  neighbour slots of every particle in the reference's
-//                    bucket order, four per block (block b of all particles
-//                    contiguous, so a warp reads four 128-byte lines per
-//                    block); the last block's entries past the count are p
-//                    (nbr_entry, nbr_block)
+//   nbr[15][n] uint4 neighbour lists in the reference's bucket order, one
+//                    16-byte block of consecutive entries per particle and
+//                    block index (column p, so a warp reads four 128-byte
+//                    lines per block): eight 16-bit offsets into the record
+//                    tile of the particle's block of kTileSlots slots
+//                    (TileInfo), or four 32-bit slots where the block has no
+//                    tile; the last block's entries past the count are the
+//                    particle itself
 //   ncount[n] u8     bucket sizes
 //   cstart[C+1] u32  start slot of every cell (lower bound), cstart[C] = n
 //
@@ -42,15 +45,6 @@ namespace sphpc {
 
 constexpr int kMaxNeighbors = 60;   // MAX_NEIGHBORS, neighbors.h:6
 
-// 32-byte record for the post-solve passes that gather a second quantity of
-// each neighbour: the 16-byte neighbour record r = {X, Y, Z, w} and a float4
-// e (colour gradient, or velocity), so a neighbour costs one 256-bit gather
-// instead of two 128-bit ones.
-struct __align__(32) NV {
-  uint4 r;
-  float4 e;
-};
-
 // Position record of one particle: step-start x and displacement d = x* - x.
 struct __align__(32) PD {
   float4 x;
@@ -59,9 +53,15 @@ struct __align__(32) PD {
 
 // Packed FP32x2 (sm_100): two independent IEEE single-precision operations
 // per instruction, each rounded to nearest as its scalar form.
-__device__ __forceinline__ uint64_t f2_dup(float a) {
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
   uint64_t r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_dup(float a) { return f2_pack(a, a); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
@@ -120,6 +120,7 @@ enum : uint32_t {
   kErrCellRange = 1u << 2,         // a particle hashed outside the grid
   kErrScanSpin = 1u << 3,
   kErrNbrTail = 1u << 5,           // a list block's entries past the count are not p
+  kErrTileWait = 1u << 6,          // the wait for a tile's bulk copies gave up
 };
 
 struct DevParams {
@@ -139,6 +140,7 @@ struct DevParams {
   // neighbour-build FP32 pre-test band: pairs with FP32 r^2 in [lo, hi] go
   // to the exact FP64 test (lo = -1, hi = inf: every pair does)
   float bld_h2lo, bld_h2hi;
+  float bld_band;       // the band's half width (inf: every pair)
   float h, h2;
   float rmin;           // r floor 1e-4 h (particles.c:636)
   // smoothing-kernel constants; *_m variants carry the particle mass
@@ -174,11 +176,32 @@ struct DevParams {
   float model_to_world;
 };
 
+// The neighbourhood of kTileSlots consecutive slots as nine contiguous slot
+// ranges: with k0 and k1 the cell keys of the first and the last slot, range
+// r = 3 (dz + 1) + dy + 1 holds the cells k0 + d - 1 .. k1 + d + 1, d = dz nx ny
+// + dy nx, so it covers cells cx-1 .. cx+1 of that row for every slot of the
+// block, also where the block runs over the end of a row of cells.  Range r
+// starts at slot s[r] and at record o[r] of the tile that holds all nine one
+// after the other (total records; -1: more than kTileCap, or a particle whose
+// neighbour cells are not the regular ones: the block's lists hold slots).
+// Range starts and lengths are even, so that pairs of slots stay together.
+//
+// kTileCap: nine ranges of 128 slots and about four cells at the ends hold 1400
+// records at the rest density; 1472 records of 16 bytes leave room for nine
+// blocks per SM.
+constexpr int kTileSlots = 128;
+constexpr int kTileCap = 1472;
+struct TileInfo {
+  int s[9], o[9], total, pad;
+};
+
 // View of the per-step neighbour structure.
 struct NbrView {
-  const uint32_t* __restrict__ nbr;     // [kMaxNeighbors / 4][n] blocks of 4 entries
+  const uint32_t* __restrict__ nbr;     // [15][n] blocks of 16 bytes
   const uint8_t* __restrict__ ncount;   // [n]
   const uint32_t* __restrict__ cstart;  // [C+1]
+  const TileInfo* __restrict__ tiles;   // [ceil(n / kTileSlots)]
+  uint32_t* err;
   int n;
   int nx, ny, nz;
   uint32_t nxny;
@@ -193,123 +216,162 @@ __device__ __forceinline__ void unpack_cell(const NbrView& v, uint32_t cp, int& 
   cz = (int)(cp >> (v.bx + v.by));
 }
 
-// Neighbour lists, nbr4[15][n] (uint4): block b of particle p holds its list
-// entries 4b .. 4b+3 (column b of all particles contiguous, so a warp reads
-// four whole 128-byte lines per block index); the entries of the last block
-// past the count hold p itself.  Entry j of particle p:
-__device__ __forceinline__ uint32_t nbr_entry(const NbrView& v, int p, int j) {
-  return __ldg(v.nbr + (((size_t)(j >> 2) * v.n + p) << 2) + (j & 3));
-}
 __device__ __forceinline__ uint4 nbr_block(const NbrView& v, int p, int b) {
   return __ldg(reinterpret_cast<const uint4*>(v.nbr) + (size_t)b * v.n + p);
 }
 
-// Visits the neighbour slots of particle p in the reference's bucket order
-// (FillNeighbors, neighbors.c:247-295: dz, dy, dx, then ascending sorted
-// index), as stored by the neighbour build.
-template <class F>
-__device__ __forceinline__ void for_each_neighbor(const NbrView& v, int p, F&& f) {
-  const int cnt = (int)__ldg(v.ncount + p);
-#pragma unroll 2
-  for (int j = 0; j < cnt; ++j) f((int)nbr_entry(v, p, j));
+__device__ __forceinline__ bool has_tile(const NbrView& v, int p) {
+  return __ldg(&v.tiles[p / kTileSlots].total) >= 0;
 }
 
-// The batched visits below take a batch of four list entries per 128-bit
-// load (one block) and load the next block before the bodies of this batch
-// run, so a batch waits only for its record gathers (the list read from HBM
-// overlaps the previous batch).  The entries of the last block past the count
-// are p: those slots load the particle's own record and are skipped, or, with
-// kPadSlots, visited as the pair (p, p) (for bodies whose every term carries
-// the pair difference, which is 0).
-#define SPHPC_NBR_BATCH_HEAD                                      \
-  static_assert(B == 4, "a batch is one four-entry list block"); \
-  const int cnt = (int)__ldg(v.ncount + p);                      \
-  uint4 blk = cnt > 0 ? nbr_block(v, p, 0) : make_uint4(p, p, p, p)
-#define SPHPC_NBR_BATCH_NEXT(j0)                                                         \
-  const int q[4] = {(int)blk.x, (int)blk.y, (int)blk.z, (int)blk.w};                    \
-  if ((j0) + 4 < cnt) blk = nbr_block(v, p, ((j0) >> 2) + 1)
+// Slot of list entry j of particle p (entry by entry: for exports and checks).
+__device__ __forceinline__ uint32_t nbr_entry(const NbrView& v, int p, int j) {
+  if (!has_tile(v, p)) return __ldg(v.nbr + (((size_t)(j >> 2) * v.n + p) << 2) + (j & 3));
+  const uint16_t* l = reinterpret_cast<const uint16_t*>(v.nbr);
+  const int i = (int)(__ldg(l + (((size_t)(j >> 3) * v.n + p) << 3) + (j & 7)) >> 4);
+  const TileInfo* t = v.tiles + p / kTileSlots;
+  int r = 8;
+  while (r > 0 && __ldg(&t->o[r]) > i) --r;
+  return (uint32_t)(__ldg(&t->s[r]) + i - __ldg(&t->o[r]));
+}
 
-// Each neighbour's 16-byte record loaded for f(q, rq).
-template <int B, bool kPadSlots = false, class F>
-__device__ __forceinline__ void for_each_neighbor_nr(const NbrView& v, const uint4* __restrict__ nr,
-                                                     int p, F&& f) {
-  SPHPC_NBR_BATCH_HEAD;
-  for (int j0 = 0; j0 < cnt; j0 += 4) {
-    SPHPC_NBR_BATCH_NEXT(j0);
-    uint4 r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) r[u] = ld_nr(nr, q[u]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (kPadSlots || j0 + u < cnt) f(q[u], r[u]);
+// ---------------------------------------------------------------------------
+// Tiles in shared memory.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// Bounded wait for phase 0 of an mbarrier (~1e6 polls, each of which may
+// itself suspend the thread for a while).
+__device__ __forceinline__ bool mbar_wait0(uint64_t* mbar) {
+  const uint32_t addr = smem_addr(mbar);
+  for (int i = 0; i < (1 << 20); ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred P1;\nmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], 0;\n"
+        "selp.b32 %0, 1, 0, P1;\n}\n"
+        : "=r"(ok)
+        : "r"(addr)
+        : "memory");
+    if (ok) return true;
   }
+  return false;
 }
 
-// The same batched visit with the whole batch handed to f(r[B], nvalid):
-// r[u] is the record of list entry j0 + u for u < nvalid = min(B, cnt - j0)
-// and the particle's own record past the count (the pair (p, p), difference
-// 0), so a body can combine the batch's terms before adding them to a sum.
-template <int B, class F>
-__device__ __forceinline__ void for_each_batch_nr(const NbrView& v, const uint4* __restrict__ nr,
-                                                  int p, F&& f) {
-  SPHPC_NBR_BATCH_HEAD;
-  for (int j0 = 0; j0 < cnt; j0 += 4) {
-    SPHPC_NBR_BATCH_NEXT(j0);
-    uint4 r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) r[u] = ld_nr(nr, q[u]);
-    f(r, cnt - j0);
-  }
+__device__ __forceinline__ void mbar_init1(uint64_t* mbar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mbar)));
+  asm volatile("fence.mbarrier_init.release.cluster;");
 }
 
-__device__ __forceinline__ void ld_nv(const NV* __restrict__ base, int i, uint4& r, float4& e) {
-  asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-      : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w), "=f"(e.x), "=f"(e.y), "=f"(e.z), "=f"(e.w)
-      : "l"(base + i));
-}
-
-__device__ __forceinline__ void st_nv(NV* base, int i, const uint4 r, const float4 e) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(base + i), "r"(r.x),
-               "r"(r.y), "r"(r.z), "r"(r.w), "f"(e.x), "f"(e.y), "f"(e.z), "f"(e.w)
+__device__ __forceinline__ void mbar_expect(uint64_t* mbar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)),
+               "r"(bytes)
                : "memory");
 }
 
-// Batched visit over the 32-byte records {r, e}: f(q, rq, eq), as
-// for_each_neighbor_nr with one 256-bit gather per neighbour.
-template <int B, bool kPadSlots = false, class F>
-__device__ __forceinline__ void for_each_neighbor_nv(const NbrView& v, const NV* __restrict__ nv,
-                                                     int p, F&& f) {
-  SPHPC_NBR_BATCH_HEAD;
-  for (int j0 = 0; j0 < cnt; j0 += 4) {
-    SPHPC_NBR_BATCH_NEXT(j0);
-    uint4 r[4];
-    float4 e[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) ld_nv(nv, q[u], r[u], e[u]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (kPadSlots || j0 + u < cnt) f(q[u], r[u], e[u]);
-  }
+// One bulk copy to this block's shared memory (16-byte aligned, a multiple of
+// 16 bytes), counted on mbar.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
+                                          uint64_t* mbar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(smem_addr(dst)),
+      "l"(src), "r"(bytes), "r"(smem_addr(mbar))
+      : "memory");
 }
 
-// Batched visit over the 32-byte particle records with the batch handed to
-// f(x[B], d[B], nvalid), nvalid = min(B, cnt - j0); slots past the count
-// hold the particle's own record and are the body's to skip.
-template <int B, class F>
-__device__ __forceinline__ void for_each_batch_pd(const NbrView& v, const PD* __restrict__ pd,
-                                                  int p, F&& f) {
-  SPHPC_NBR_BATCH_HEAD;
-  for (int j0 = 0; j0 < cnt; j0 += 4) {
-    SPHPC_NBR_BATCH_NEXT(j0);
-    float4 x[4], d[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) ld_pd(pd, q[u], x[u], d[u]);
-    f(x, d, cnt - j0);
+// The tile of a block of kTileSlots threads: tile_load starts the copies of
+// NARR arrays of 16-byte records (array k at byte k * kTileCap * 16 of `tile`)
+// and returns whether the block has a tile; tile_wait waits for them.  Every
+// thread of the block calls both.
+template <int NARR>
+__device__ __forceinline__ bool tile_load(const NbrView& v, const void* a0, const void* a1,
+                                          unsigned char* tile, uint64_t* mbar) {
+  const TileInfo* t = v.tiles + blockIdx.x;
+  const int total = __ldg(&t->total);
+  if (total >= 0 && threadIdx.x < 32) {
+    const int r = threadIdx.x;
+    int s = 0, o = 0, e = 0;
+    if (r < 9) {
+      s = __ldg(&t->s[r]);
+      o = __ldg(&t->o[r]);
+      e = r < 8 ? __ldg(&t->o[r + 1]) : total;
+    }
+    if (r == 0) {
+      mbar_init1(mbar);
+      mbar_expect(mbar, (uint32_t)total * (16u * NARR));
+    }
+    __syncwarp();
+    if (e > o) {
+      const uint32_t bytes = (uint32_t)(e - o) * 16u;
+      bulk_load(tile + o * 16, static_cast<const uint4*>(a0) + s, bytes, mbar);
+      if (NARR == 2)
+        bulk_load(tile + (kTileCap + o) * 16, static_cast<const uint4*>(a1) + s, bytes, mbar);
+    }
   }
+  return total >= 0;
 }
 
-#undef SPHPC_NBR_BATCH_HEAD
-#undef SPHPC_NBR_BATCH_NEXT
+__device__ __forceinline__ bool tile_wait(const NbrView& v, bool tiled, uint64_t* mbar) {
+  if (!tiled) return true;
+  __syncthreads();  // the mbarrier is initialised
+  if (mbar_wait0(mbar)) return true;
+  atomicOr(v.err, kErrTileWait);
+  mbar_wait0(mbar);  // the copies in flight write this block's shared memory
+  return false;
+}
+
+// A batch of four list entries: the neighbours' records and, with a second
+// array, their vectors; entries past the count are the particle itself (the
+// pair (p, p): difference 0).
+template <int NARR>
+struct Batch {
+  uint4 r[4];
+  float4 e[NARR == 2 ? 4 : 1];
+};
+
+// Visits the list of particle p in batches of four: f(batch, nvalid) with
+// nvalid = count - (entries before the batch).  tiled: offsets into the tile
+// (16-bit entries, eight per block), else slots (gathered from nr and e).  The
+// next list block is loaded before this one's bodies run.  (Eight entries a
+// round without the test between them measured 5% slower: more registers live
+// for no fewer wavefronts.)
+template <int NARR, class F>
+__device__ __forceinline__ void visit(const NbrView& v, bool tiled, const unsigned char* tile,
+                                      const uint4* __restrict__ nr, const float4* __restrict__ e,
+                                      int p, int cnt, uint4 blk, F&& f) {
+  if (tiled) {
+    auto load = [&](uint32_t w0, uint32_t w1) {
+      const uint32_t o[4] = {w0 & 0xffffu, w0 >> 16, w1 & 0xffffu, w1 >> 16};
+      Batch<NARR> b;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        b.r[u] = *reinterpret_cast<const uint4*>(tile + o[u]);
+        if (NARR == 2) b.e[u] = *reinterpret_cast<const float4*>(tile + kTileCap * 16 + o[u]);
+      }
+      return b;
+    };
+    for (int j0 = 0; j0 < cnt; j0 += 8) {
+      const uint4 w = blk;
+      if (j0 + 8 < cnt) blk = nbr_block(v, p, (j0 >> 3) + 1);
+      f(load(w.x, w.y), cnt - j0);
+      if (j0 + 4 < cnt) f(load(w.z, w.w), cnt - j0 - 4);
+    }
+  } else {
+    for (int j0 = 0; j0 < cnt; j0 += 4) {
+      const int q[4] = {(int)blk.x, (int)blk.y, (int)blk.z, (int)blk.w};
+      if (j0 + 4 < cnt) blk = nbr_block(v, p, (j0 >> 2) + 1);
+      Batch<NARR> b;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        b.r[u] = ld_nr(nr, q[u]);
+        if (NARR == 2) b.e[u] = __ldg(e + q[u]);
+      }
+      f(b, cnt - j0);
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Canonical double predicted position and the reference's box clamp.
