@@ -23,7 +23,7 @@ int SortByKey(unsigned int *const keys, unsigned int *const values, const int co
  * callers that must not allocate device memory (a host that owns all device
  * memory through its own pool, or a time-critical loop where a cudaMalloc,
  * which can synchronise the device or fail under memory pressure, is not
- * acceptable).  Its scratch is a fixed array of about 2.4 MB inside the
+ * acceptable).  Its scratch is a fixed array of about 3.2 MB inside the
  * library, held by every GPU that loads the library until the process exits,
  * so count is limited to 262,144 pairs (larger counts return SPHPC_EINVAL).
  * It calls no cudaMalloc or cudaFree.  The first call on a device, and the

@@ -657,17 +657,27 @@ void launch_reorder(const DevParams& P, const uint32_t* sorted_ids, const uint32
                                               move_vel ? 1 : 0, ex);
 }
 
-void launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint32_t* cstart,
-                        uint4* gaps, uint32_t* gap_count, uint32_t* err, cudaStream_t st) {
+// Up to kBoundsMaxCells cells the bounds kernel writes the table in one launch
+// (two blocks per SM and one wave); beyond, its search per 1024 cells costs
+// more than the worklist's second launch.
+constexpr uint32_t kBoundsMaxCells = 1u << 19;
+
+int launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint32_t* cstart,
+                       uint4* gaps, uint32_t* gap_count, uint32_t* err, cudaStream_t st) {
   if (n == 0) {
     cudaMemsetAsync(cstart, 0, sizeof(uint32_t) * ((size_t)ncells + 1), st);
-    return;
+    return 0;
+  }
+  if (ncells <= kBoundsMaxCells) {
+    launch_bounds(keys_sorted, n, (int)ncells + 1, cstart, false, st);
+    return 1;
   }
   cudaMemsetAsync(gap_count, 0, sizeof(uint32_t), st);
   const int threads = (n + kStartsPerThread - 1) / kStartsPerThread;
   k_cell_starts<<<grid_for(threads), kBlock, 0, st>>>(keys_sorted, n, ncells, cstart, gaps,
                                                        gap_count, err);
   k_fill_gaps<<<148 * 16, kBlock, 0, st>>>(gaps, gap_count, cstart);
+  return 2;
 }
 
 void launch_build_neighbors(const DevParams& P, const NbrView& V, const PD* pd,

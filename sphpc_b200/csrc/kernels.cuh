@@ -47,7 +47,8 @@ void launch_reorder(const DevParams& P, const uint32_t* sorted_ids, const uint32
 // Cell start table cstart[0..C] from sorted keys (lower bounds; cstart[C]=n).
 // gaps: worklist scratch of >= n + 2 + C/4096 + 2 uint4 entries; gap_count:
 // one u32.
-void launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint32_t* cstart,
+// Returns the kernels launched.
+int launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint32_t* cstart,
                         uint4* gaps, uint32_t* gap_count, uint32_t* err, cudaStream_t st);
 
 // Neighbour build (FillNeighbors, neighbors.c:217-298): per particle, its

@@ -137,14 +137,13 @@ __device__ __forceinline__ uint64_t h_minus_r(const DevParams& P, uint64_t r2c, 
 
 // The same in fixed-point units (r2f = |d|^2 of the record difference):
 // r2c = max(r2f, r_min^2) and rinv_f = 2^-k / r, so the loops need no
-// rescaling of r^2; r_f = r 2^k is r2c rinv (fx_r), and h_f - r_f, floored at
+// rescaling of r^2; r_f = r 2^k is r2c rinv, and h_f - r_f, floored at
 // 0, one fused multiply-add (fx_hm).
 __device__ __forceinline__ void floored_r_fx(const DevParams& P, float r2f, float& r2c,
                                              float& rinv) {
   r2c = fmaxf(r2f, P.rmin2_fx);
   rinv = rsqrt_normal(r2c);
 }
-__device__ __forceinline__ float fx_r(float r2c, float rinv) { return __fmul_rn(r2c, rinv); }
 __device__ __forceinline__ float fx_hm(const DevParams& P, float r2c, float rinv) {
   return fmaxf(fmaf(-r2c, rinv, P.h_fx), 0.0f);
 }

@@ -1,6 +1,7 @@
 // radix_sort.cu -- onesweep LSD radix sort and the cell-bounds seam kernels.
 #include "radix_sort.cuh"
 
+#include <climits>
 #include <vector>
 
 namespace sphpc {
@@ -29,32 +30,19 @@ __global__ void __launch_bounds__(256) k_digit_histogram(const uint32_t* __restr
   __shared__ uint32_t s_hist[kMaxPasses * kRadix];
   for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    count_key_digits(s_hist, __ldg(keys + i), passes);
+  const int step = gridDim.x * blockDim.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i < n - 3 * step; i += 4 * step) {
+    uint32_t k[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) k[u] = __ldg(keys + i + u * step);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) count_key_digits(s_hist, k[u], passes);
+  }
+  for (; i < n; i += step) count_key_digits(s_hist, __ldg(keys + i), passes);
   __syncthreads();
   for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x)
     if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
-}
-
-// Exclusive scan of each pass's 256 digit counts (one block, 256 threads).
-__global__ void __launch_bounds__(256) k_scan_digits(uint32_t* __restrict__ hist, int passes) {
-  __shared__ uint32_t s_warp[kRadix / 32];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int p = 0; p < passes; ++p) {
-    const uint32_t v = hist[p * kRadix + t];
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    uint32_t wsum = 0;
-    for (int w = 0; w < warp; ++w) wsum += s_warp[w];
-    hist[p * kRadix + t] = wsum + x - v;
-    __syncthreads();
-  }
 }
 
 // One digit pass.  vals_in == nullptr means the values are the input
@@ -63,42 +51,59 @@ __global__ void __launch_bounds__(256) k_scan_digits(uint32_t* __restrict__ hist
 // each) rather than the two that the compiler's own choice of 128
 // registers leaves room for: the passes wait on loads and on the
 // look-back, so resident warps are what hides it.  The values are loaded
-// only when the tile is staged, which is what lets the ranking fit.
-__global__ void __launch_bounds__(kSortThreads, 5)
+// only when the tile is staged, which is what lets the ranking fit.  The
+// smaller tiles take eight blocks.  The digits' offsets are scanned from the
+// counts in every block (256 values: less than a launch), and a digit that
+// all keys share leaves the order as it is: its tiles are copied.
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 5 : 8)
     k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n,
-               int shift, const uint32_t* __restrict__ digit_offset,
+               int shift, const uint32_t* __restrict__ digit_count,
                uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_counter,
                uint32_t* __restrict__ err, int spin_limit) {
+  constexpr int kSortTile = kSortThreads * ITEMS;
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_whist[kSortWarps][kRadix + 1];
   __shared__ uint32_t s_dstart[kRadix];
   __shared__ uint32_t s_gbase[kRadix];
-  __shared__ uint32_t s_wsum[kRadix / 32];
+  __shared__ uint32_t s_wsum[kRadix / 32], s_gsum[kRadix / 32];
   __shared__ uint32_t s_keys[kSortTile];
   __shared__ uint32_t s_vals[kSortTile];
 
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t all = __ldg(digit_count + t);
   if (t == 0) s_tile = atomicAdd(tile_counter, 1u);
   for (int i = t; i < kSortWarps * (kRadix + 1); i += kSortThreads)
     (&s_whist[0][0])[i] = 0;
-  __syncthreads();
+  const bool one_digit = __syncthreads_or(all == (uint32_t)n) != 0;
   const uint32_t tile = s_tile;
   // n <= kLbValue < 2^30, so every index fits 32 bits
   const int tile_base = (int)tile * kSortTile;
-  const int wbase = tile_base + warp * 32 * kSortItems;
+  if (one_digit) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int idx = tile_base + i * kSortThreads + t;
+      if (idx < n) {
+        keys_out[idx] = __ldg(keys_in + idx);
+        vals_out[idx] = vals_in ? __ldg(vals_in + idx) : (uint32_t)idx;
+      }
+    }
+    return;
+  }
+  const int wbase = tile_base + warp * 32 * ITEMS;
 
   // the values are loaded only when the tile is staged, so that the ranking
   // holds two arrays of registers, not three
-  uint32_t key[kSortItems], rank[kSortItems];
+  uint32_t key[ITEMS], rank[ITEMS];
 #pragma unroll
-  for (int i = 0; i < kSortItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const int idx = wbase + i * 32 + lane;
     key[i] = idx < n ? __ldg(keys_in + idx) : 0xffffffffu;
   }
   const uint32_t lt = lanemask_lt();
 #pragma unroll
-  for (int i = 0; i < kSortItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const int idx = wbase + i * 32 + lane;
     const uint32_t d = idx < n ? ((key[i] >> shift) & (kRadix - 1)) : (uint32_t)kRadix;
     const uint32_t peers = __match_any_sync(0xffffffffu, d);
@@ -166,25 +171,36 @@ __global__ void __launch_bounds__(kSortThreads, 5)
       }
       st_volatile(my, kLbInc | (excl + cnt));
     }
-    s_gbase[d] = __ldg(digit_offset + d) + excl;
-    // tile-local exclusive scan of cnt over digits
-    uint32_t x = cnt;
+    // exclusive scans over the digits: of the tile's counts, and of the counts
+    // of all keys
+    uint32_t x = cnt, g = all;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const uint32_t z = __shfl_up_sync(0xffffffffu, g, o);
+      if (lane >= o) {
+        x += y;
+        g += z;
+      }
     }
-    if (lane == 31) s_wsum[warp] = x;
+    if (lane == 31) {
+      s_wsum[warp] = x;
+      s_gsum[warp] = g;
+    }
     __syncthreads();
-    uint32_t wsum = 0;
-    for (int w = 0; w < warp; ++w) wsum += s_wsum[w];
+    uint32_t wsum = 0, gsum = 0;
+    for (int w = 0; w < warp; ++w) {
+      wsum += s_wsum[w];
+      gsum += s_gsum[w];
+    }
     s_dstart[d] = wsum + x - cnt;
+    s_gbase[d] = gsum + g - all + excl;
   }
   __syncthreads();
 
   // Stage the tile in digit order.
 #pragma unroll
-  for (int i = 0; i < kSortItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const int idx = wbase + i * 32 + lane;
     if (idx < n) {
       const uint32_t d = (key[i] >> shift) & (kRadix - 1);
@@ -196,7 +212,7 @@ __global__ void __launch_bounds__(kSortThreads, 5)
   __syncthreads();
   const int valid = min(kSortTile, n - tile_base);
 #pragma unroll
-  for (int i = 0; i < kSortItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const int k = t + i * kSortThreads;
     if (k < valid) {
       const uint32_t kk = s_keys[k];
@@ -212,20 +228,87 @@ __global__ void __launch_bounds__(kSortThreads, 5)
   }
 }
 
-__global__ void k_bounds(const uint32_t* __restrict__ keys, int n, int count,
-                         uint32_t* __restrict__ out, int upper) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < count;
-       c += gridDim.x * blockDim.x) {
-    int lo = 0, hi = n;
-    const uint32_t v = (uint32_t)c;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      const uint32_t k = __ldg(keys + mid);
-      const bool go_right = upper ? (k <= v) : (k < v);
-      if (go_right) lo = mid + 1; else hi = mid;
-    }
-    out[c] = (uint32_t)lo;
+// First position of sorted keys[0, n) whose key is >= v, by the whole warp: 32
+// probes per step.
+__device__ int warp_lower_bound(const uint32_t* __restrict__ keys, int n, int64_t v) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = n;  // keys before lo are < v, keys from hi on are >= v
+  while (lo < hi) {
+    const int step = (hi - lo + 31) / 32;
+    const int at = lo + lane * step;
+    const bool less = at < hi && (int64_t)__ldg(keys + at) < v;
+    const int below = __popc(__ballot_sync(0xffffffffu, less));
+    if (below == 0) break;
+    const int last = lo + (below - 1) * step;  // the last probe below v
+    hi = min(hi, last + step);
+    lo = last + 1;
   }
+  return lo;
+}
+
+// start[c] = lower_bound(keys, first + c) of cells c in [0, count).  A block
+// takes kBoundCells cells: two warps find where their keys begin and end, the
+// block reads those keys once, marks the first key of each cell, and a suffix
+// minimum over the cells gives the starts of the empty ones.  A run of more than
+// kBoundRange keys is searched cell by cell instead.  Bounds: the latency of the
+// two searches (four dependent loads at 1M keys).  1.8M cells over 1M keys, cold
+// caches: 38 us with a binary search of all keys per cell, 20 us so.
+constexpr int kBoundPer = 8;
+constexpr int kBoundCells = 256 * kBoundPer;
+constexpr int kBoundRange = 1 << 15;
+__global__ void __launch_bounds__(256)
+    k_bounds(const uint32_t* __restrict__ keys, int n, int count, int first,
+             uint32_t* __restrict__ out) {
+  __shared__ int s_first[kBoundCells];
+  __shared__ int s_range[2], s_min[8];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int c0 = blockIdx.x * kBoundCells;
+  const int nc = min(kBoundCells, count - c0);
+  const int64_t v0 = (int64_t)c0 + first;
+  if (warp < 2) {
+    const int b = warp_lower_bound(keys, n, v0 + (warp ? nc : 0));
+    if (lane == 0) s_range[warp] = b;
+  }
+  for (int i = t; i < kBoundCells; i += 256) s_first[i] = INT_MAX;
+  __syncthreads();
+  const int lo = s_range[0], hi = s_range[1];
+  if (hi - lo > kBoundRange) {
+    for (int i = t; i < nc; i += 256) {
+      int a = lo, b = hi;
+      while (a < b) {
+        const int mid = (a + b) >> 1;
+        if ((int64_t)__ldg(keys + mid) < v0 + i) a = mid + 1; else b = mid;
+      }
+      out[c0 + i] = (uint32_t)a;
+    }
+    return;
+  }
+  for (int j = lo + t; j < hi; j += 256) {
+    const uint32_t k = __ldg(keys + j);
+    if (j == lo || __ldg(keys + j - 1) != k) s_first[(int64_t)k - v0] = j;
+  }
+  __syncthreads();
+  // suffix minimum: kBoundPer cells per thread, then over the lanes and the warps
+  int m[kBoundPer];
+#pragma unroll
+  for (int u = 0; u < kBoundPer; ++u) m[u] = s_first[kBoundPer * t + u];
+#pragma unroll
+  for (int u = kBoundPer - 2; u >= 0; --u) m[u] = min(m[u], m[u + 1]);
+  int x = m[0];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_down_sync(0xffffffffu, x, o);
+    if (lane + o < 32) x = min(x, y);
+  }
+  if (lane == 0) s_min[warp] = x;
+  int after = __shfl_down_sync(0xffffffffu, x, 1);
+  if (lane == 31) after = INT_MAX;
+  __syncthreads();
+  for (int w = warp + 1; w < 8; ++w) after = min(after, s_min[w]);
+  after = min(after, hi);
+#pragma unroll
+  for (int u = 0; u < kBoundPer; ++u)
+    if (kBoundPer * t + u < nc) out[c0 + kBoundPer * t + u] = (uint32_t)min(m[u], after);
 }
 
 }  // namespace
@@ -233,9 +316,17 @@ __global__ void k_bounds(const uint32_t* __restrict__ keys, int n, int count,
 void launch_digit_histogram(const uint32_t* keys, int n, int passes, uint32_t* hist,
                             cudaStream_t stream) {
   if (n <= 0) return;
-  int blocks = (n + 255) / 256;
+  // 4096 keys a block: fewer would spend their time adding 256 counts per
+  // digit to the totals (1M keys: 12 us with 256 threads per 885 keys)
+  int blocks = (n + 4095) / 4096;
   if (blocks > 148 * 8) blocks = 148 * 8;
   k_digit_histogram<<<blocks, 256, 0, stream>>>(keys, n, passes, hist);
+}
+
+cudaError_t sort_clear(const SortScratch& s, int n, int passes, cudaStream_t stream) {
+  const size_t words = (size_t)kMaxPasses * kRadix + kMaxPasses +
+                       (size_t)passes * sort_tiles(n > 0 ? n : 1) * kRadix;
+  return cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * words, stream);
 }
 
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, int n, int passes,
@@ -256,26 +347,22 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, int n, int passes,
   }
   const int tiles = sort_tiles(n);
   if (!hist_ready) {
-    e = cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, stream);
+    e = sort_clear(s, n, passes, stream);
     if (e != cudaSuccess) return e;
     launch_digit_histogram(keys, n, passes, s.hist, stream);
   }
-  e = cudaMemsetAsync(s.lookback, 0, sizeof(uint32_t) * (size_t)passes * tiles * kRadix,
-                      stream);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(s.counters, 0, sizeof(uint32_t) * kMaxPasses, stream);
-  if (e != cudaSuccess) return e;
-  k_scan_digits<<<1, kRadix, 0, stream>>>(s.hist, passes);
   // Pass p reads the previous output and writes buffer set (p & 1):
   // set 0 = scratch alternates, set 1 = the caller's arrays.
   uint32_t* const bk[2] = {s.keys_alt, keys};
   uint32_t* const bv[2] = {s.vals_alt, vals};
   const uint32_t* kin = keys;
   const uint32_t* vin = vals_iota ? nullptr : vals;
+  const int items = sort_items(n);
   for (int p = 0; p < passes; ++p) {
     uint32_t* kout = bk[p & 1];
     uint32_t* vout = bv[p & 1];
-    k_onesweep<<<tiles, kSortThreads, 0, stream>>>(
+    auto kernel = items == 4 ? k_onesweep<4> : items == 8 ? k_onesweep<8> : k_onesweep<16>;
+    kernel<<<tiles, kSortThreads, 0, stream>>>(
         kin, vin, kout, vout, n, p * kRadixBits, s.hist + p * kRadix,
         s.lookback + (size_t)p * tiles * kRadix, s.counters + p, s.err, kSpinLimit);
     kin = kout;
@@ -302,20 +389,14 @@ cudaError_t lookback_wait_probe(int spin_limit, uint32_t* err_bits) {
   // Two tiles of keys; the tile counter starts at 1, so the one CTA
   // launched ranks tile 1 and looks back at tile 0, whose flag no CTA ever
   // writes.  Its wait gives up after spin_limit polls and sets kErrSortSpin;
-  // the digit offsets are those of all 2 tiles, so every scatter the CTA
+  // the digit counts are those of both tiles, so every scatter the CTA
   // then makes stays below n.
-  const int n = 2 * kSortTile;
+  constexpr int kItems = 16, n = 2 * kSortThreads * kItems;
   std::vector<uint32_t> hk(n);
   uint32_t hist[kRadix] = {};
   for (int i = 0; i < n; ++i) {
     hk[i] = (uint32_t)i * 2654435761u;
     ++hist[hk[i] & (kRadix - 1)];
-  }
-  uint32_t offs[kRadix];
-  uint32_t acc = 0;
-  for (int d = 0; d < kRadix; ++d) {
-    offs[d] = acc;
-    acc += hist[d];
   }
   uint32_t* buf = nullptr;
   const size_t words = 4 * (size_t)n + kRadix + 2 * kRadix + 2;
@@ -333,10 +414,10 @@ cudaError_t lookback_wait_probe(int spin_limit, uint32_t* err_bits) {
   e = cudaMemset(buf, 0, words * sizeof(uint32_t));
   if (e == cudaSuccess)
     e = cudaMemcpy(keys, hk.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(doff, offs, sizeof(offs), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(doff, hist, sizeof(hist), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(counter, &one, sizeof(one), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    k_onesweep<<<1, kSortThreads>>>(keys, vals, kout, vout, n, 0, doff, lookback, counter, err,
+    k_onesweep<kItems><<<1, kSortThreads>>>(keys, vals, kout, vout, n, 0, doff, lookback, counter, err,
                                     spin_limit);
     e = cudaGetLastError();
   }
@@ -349,9 +430,9 @@ cudaError_t lookback_wait_probe(int spin_limit, uint32_t* err_bits) {
 cudaError_t launch_bounds(const uint32_t* keys, int n, int count, uint32_t* out, bool upper,
                           cudaStream_t stream) {
   if (count <= 0) return cudaSuccess;
-  int blocks = (count + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  k_bounds<<<blocks, 256, 0, stream>>>(keys, n, count, out, upper ? 1 : 0);
+  // the upper bound of c is the lower bound of c + 1
+  const int blocks = (int)(((int64_t)count + kBoundCells - 1) / kBoundCells);
+  k_bounds<<<blocks, 256, 0, stream>>>(keys, n, count, upper ? 1 : 0, out);
   return cudaGetLastError();
 }
 

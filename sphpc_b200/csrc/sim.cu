@@ -206,12 +206,9 @@ class DeviceSim {
     SPHPC_RC(dalloc(&resid, 16));
     SPHPC_RC(dalloc(&sort.keys_alt, c));
     SPHPC_RC(dalloc(&sort.vals_alt, c));
-    const size_t aux = sort_aux_words(c) + 4;
+    const size_t aux = sort_aux_words(c);
     SPHPC_RC(dalloc(&sort_aux, aux));
-    sort.hist = sort_aux;
-    sort.counters = sort_aux + (size_t)kMaxPasses * kRadix;
-    sort.err = sort_aux + (size_t)kMaxPasses * kRadix + kMaxPasses;
-    sort.lookback = sort_aux + (size_t)kMaxPasses * kRadix + kMaxPasses + 4;
+    sort_layout(sort, sort_aux);
     SPHPC_CK(cudaMemsetAsync(small, 0, 8 * sizeof(uint32_t), stream));
     SPHPC_CK(cudaMemsetAsync(sort_aux, 0, aux * sizeof(uint32_t), stream));
     SPHPC_CK(cudaMemsetAsync(pd, 0, sizeof(PD) * c, stream));
@@ -543,7 +540,7 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
   if (!grid_ready) return set_error(SPHPC_ENOTREADY, "neighbour grid not initialised");
   {
     Scope sc(this, "hash");
-    SPHPC_CK(cudaMemsetAsync(sort.hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, stream));
+    SPHPC_CK(sort_clear(sort, n, passes, stream));
     launch_hash(P, pd, vel, ids, keys_by_id, loc_by_id, sort.hist, passes, predict, err(),
                 stream);
     launches += 1;
@@ -555,13 +552,12 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
                                            true, false, &K, &R);
     if (e != cudaSuccess)
       return set_error(SPHPC_ECUDA, "radix sort: %s", cudaGetErrorString(e));
-    launches += 1 + (unsigned)passes;
+    launches += (unsigned)passes;
   }
   keys_sorted = K;
   {
     Scope sc(this, "cell_starts");
-    launch_cell_starts(K, n, C, cstart, gaps, gap_count(), err(), stream);
-    launches += 2;
+    launches += launch_cell_starts(K, n, C, cstart, gaps, gap_count(), err(), stream);
   }
   {
     Scope sc(this, "reorder");
@@ -1932,13 +1928,10 @@ static int seam_scratch(int count, SortScratch* out) {
     sc.cap = 0;
     SPHPC_RC(dalloc(&sc.s.keys_alt, (size_t)count));
     SPHPC_RC(dalloc(&sc.s.vals_alt, (size_t)count));
-    const size_t aux = sort_aux_words(count) + 4;
+    const size_t aux = sort_aux_words(count);
     SPHPC_RC(dalloc(&sc.aux, aux));
     SPHPC_CK(cudaMemset(sc.aux, 0, aux * sizeof(uint32_t)));
-    sc.s.hist = sc.aux;
-    sc.s.counters = sc.aux + (size_t)kMaxPasses * kRadix;
-    sc.s.err = sc.aux + (size_t)kMaxPasses * kRadix + kMaxPasses;
-    sc.s.lookback = sc.aux + (size_t)kMaxPasses * kRadix + kMaxPasses + 4;
+    sort_layout(sc.s, sc.aux);
     sc.cap = count;
   }
   *out = sc.s;

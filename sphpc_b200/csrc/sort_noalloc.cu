@@ -23,13 +23,10 @@ constexpr int kNoAllocMaxPairs = 1 << 18;
 
 // Words of scratch: two alternate buffers of kNoAllocMaxPairs plus the
 // digit histograms, look-back flags, tile counters and error word of
-// radix_sort_pairs (about 2.4 MB).  Every GPU that loads the library holds
+// radix_sort_pairs (about 3.2 MB).  Every GPU that loads the library holds
 // this array until the process exits.
 constexpr size_t kNoAllocWords =
-    2 * (size_t)kNoAllocMaxPairs + ((size_t)kMaxPasses * kRadix +
-                                    (size_t)kMaxPasses * ((kNoAllocMaxPairs + kSortTile - 1) /
-                                                          kSortTile) * kRadix +
-                                    kMaxPasses) + 8;
+    2 * (size_t)kNoAllocMaxPairs + sort_aux_words(kNoAllocMaxPairs) + 8;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
@@ -131,11 +128,7 @@ extern "C" int SortByKeyNoAlloc(unsigned int* const keys, unsigned int* const va
   SortScratch s;
   s.keys_alt = base;
   s.vals_alt = base + kNoAllocMaxPairs;
-  uint32_t* aux = base + 2 * (size_t)kNoAllocMaxPairs;
-  s.hist = aux;
-  s.counters = aux + (size_t)kMaxPasses * kRadix;
-  s.err = aux + (size_t)kMaxPasses * kRadix + kMaxPasses;
-  s.lookback = aux + (size_t)kMaxPasses * kRadix + kMaxPasses + 4;
+  sort_layout(s, base + 2 * (size_t)kNoAllocMaxPairs);
   cudaStream_t st = (cudaStream_t)cuda_stream;
   // The array keeps the previous call's contents: the error word must start
   // at zero (histograms, look-back flags and tile counters are cleared by
