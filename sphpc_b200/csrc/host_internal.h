@@ -47,6 +47,10 @@ double counter_uniform01(uint64_t seed, uint64_t index, uint32_t axis);
 int sim_interleave_positions(const struct Particles* particles, double* d_out, int* n,
                              void** stream);
 
+// Unique id of the calling thread's current CUDA context (it changes when
+// cudaDeviceReset makes a new one); false when the driver cannot say.
+bool current_context_id(unsigned long long* id);
+
 // Kernel norms of SetParameters (simulation.c:173-177).
 void set_kernel_norms(Params* p);
 

@@ -28,6 +28,7 @@
 
 #include "host_internal.h"
 #include "radix_sort.cuh"
+#include "scratch.cuh"
 
 namespace sphpc {
 namespace {
@@ -451,20 +452,16 @@ extern "C" int sphpc_mesh_sdf(const float* vertices, int n_vertices, const int* 
     scale[c] = b > a ? 1024.0f / (b - a) : 0.0f;
   }
   const size_t nt = (size_t)n_triangles, nc = (nt + kCluster - 1) / kCluster;
-  // one buffer: offsets in bytes, 256-aligned
-  size_t used = 0;
-  auto part = [&](size_t bytes) {
-    const size_t at = used;
-    used += (bytes + 255) & ~(size_t)255;
-    return at;
-  };
+  ScratchLayout lay;
+  auto part = [&](size_t bytes) { return lay.part(bytes); };
   const size_t o_vert = part(12 * (size_t)n_vertices), o_tri = part(12 * nt),
                o_corner = part(36 * nt), o_key = part(4 * nt), o_order = part(4 * nt),
                o_keys2 = part(4 * nt), o_order2 = part(4 * nt), o_aux = part(4 * sort_aux_words(n_triangles)),
                o_sorted = part(48 * nc * kCluster), o_box = part(32 * nc), o_rep = part(16 * nc), o_open = part(24),
                o_step = part(4 * (size_t)total), o_phi = part(4 * (size_t)total);
-  char* buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, used);
+  CallScratch mem;
+  cudaError_t e = mem.take(lay.bytes(), 0);
+  char* buf = mem.at<char>(0);
   const SdfGrid g{dims[0], dims[1], dims[2], origin[0], origin[1], origin[2], dx};
   auto blocks = [](long long n, int per) { return (unsigned)((n + per - 1) / per); };
   if (e == cudaSuccess) {
@@ -508,7 +505,6 @@ extern "C" int sphpc_mesh_sdf(const float* vertices, int n_vertices, const int* 
     }
     if (e == cudaSuccess)
       e = cudaMemcpy(phi, d_phi, sizeof(float) * (size_t)total, cudaMemcpyDeviceToHost);
-    cudaFree(buf);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();

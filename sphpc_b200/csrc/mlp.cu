@@ -15,6 +15,7 @@
 
 #include "host_internal.h"
 #include "mlp.cuh"
+#include "scratch.cuh"
 
 namespace sphpc {
 
@@ -655,6 +656,9 @@ __global__ void k_mlp_update(const float* __restrict__ partial, int nparts,
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k > kMlpParams) return;
   double g = 0.0;
+  // 37 slices in flight: the sum waits for the loads' latency four times for
+  // 148 slices (10.4 us a launch with the compiler's unrolling, 8.4 us so)
+#pragma unroll 37
   for (int c = 0; c < nparts; ++c) g += (double)partial[(size_t)c * (kMlpParams + 1) + k];
   if (k == kMlpParams) {
     if (loss_sum) *loss_sum = (float)g;
@@ -837,21 +841,50 @@ int train_grid(int batch) {
   return tiles < 148 ? tiles : 148;
 }
 
-// Scratch of a gradient/AdamW run.
-struct TrainBufs {
-  float* partial = nullptr;
-  float* m = nullptr;
-  float* v = nullptr;
-  float* grad = nullptr;
-  float* loss = nullptr;
+// Device memory of one call on a network: its parameters, normalisation and
+// BF16 weights, a loss and an error word and room for a gradient, in one buffer
+// that one copy fills (the BF16 rounding is done here), and parts of the caller's.
+struct CallNet {
+  static constexpr size_t kNorm = (sizeof(float) * kMlpParams + 15) & ~(size_t)15;
+  static constexpr size_t kWbf = kNorm + ((sizeof(float) * kMlpNorm + 15) & ~(size_t)15);
+  static constexpr int kWeights = kMlpHidden * kMlpIn + 2 * kMlpHidden * kMlpHidden;
+  static constexpr size_t kLoss = kWbf + sizeof(__nv_bfloat16) * kWeights;  // loss, then error
+  static constexpr size_t kGrad = kLoss + 16;
+  static constexpr size_t kEnd = kGrad + sizeof(float) * kMlpParams;
+
+  ScratchLayout lay;
+  CallScratch mem;
+  MlpDevice d;
+  float *loss = nullptr, *grad = nullptr;
   uint32_t* err = nullptr;
-  ~TrainBufs() {
-    if (partial) cudaFree(partial);
-    if (m) cudaFree(m);
-    if (v) cudaFree(v);
-    if (grad) cudaFree(grad);
-    if (loss) cudaFree(loss);
-    if (err) cudaFree(err);
+
+  CallNet() { lay.part(kEnd); }
+  size_t part(size_t bytes) { return lay.part(bytes); }
+
+  int upload(const float* params, const float* norm, cudaStream_t st) {
+    SPHPC_RC(set_mlp_attrs());
+    cudaError_t e = mem.take(lay.bytes(), st);
+    if (e != cudaSuccess)
+      return set_error(SPHPC_ENOMEM, "network scratch of %zu bytes: %s", lay.bytes(),
+                       cudaGetErrorString(e));
+    alignas(16) unsigned char up[kGrad];
+    memset(up + kLoss, 0, kGrad - kLoss);
+    memcpy(up, params, sizeof(float) * kMlpParams);
+    memcpy(up + kNorm, norm, sizeof(float) * kMlpNorm);
+    __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(up + kWbf);
+    for (int off : {kOffW1, kOffW2, kOffW3}) {
+      const int n = off == kOffW1 ? kMlpHidden * kMlpIn : kMlpHidden * kMlpHidden;
+      for (int k = 0; k < n; ++k) *w++ = __float2bfloat16_rn(params[off + k]);
+    }
+    e = cudaMemcpyAsync(mem.at<char>(0), up, kGrad, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return set_error(SPHPC_ECUDA, "MLP upload: %s", cudaGetErrorString(e));
+    d.params = mem.at<float>(0);
+    d.norm = mem.at<float>(kNorm);
+    d.wbf = mem.at<__nv_bfloat16>(kWbf);
+    loss = mem.at<float>(kLoss);
+    err = mem.at<uint32_t>(kLoss + 4);
+    grad = mem.at<float>(kGrad);
+    return SPHPC_OK;
   }
 };
 
@@ -931,22 +964,16 @@ extern "C" int sphpc_mlp_forward(const float* d_feat, int n, const float* params
   if (n < 0 || !params || !norm || (n > 0 && (!d_feat || !d_out)))
     return set_error(SPHPC_EINVAL, "sphpc_mlp_forward: bad arguments");
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  MlpDevice d;
-  uint32_t* err = nullptr;
-  int rc = mlp_upload(d, params, norm, st);
-  if (!rc && cudaMalloc(&err, sizeof(uint32_t)) != cudaSuccess)
-    rc = set_error(SPHPC_ENOMEM, "sphpc_mlp_forward: error word");
+  CallNet net;
+  int rc = net.upload(params, norm, st);
   if (!rc) {
-    cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
-    launch_mlp_forward(d, d_feat, n, d_out, nullptr, nullptr, err, st);
+    launch_mlp_forward(net.d, d_feat, n, d_out, nullptr, nullptr, net.err, st);
     uint32_t h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(&h, net.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = set_error(SPHPC_ECUDA, "sphpc_mlp_forward: %s", cudaGetErrorString(e));
     else if (h) rc = set_error(SPHPC_EKERNEL, "sphpc_mlp_forward: tensor-core wait gave up (0x%x)", h);
   }
-  if (err) cudaFree(err);
-  mlp_free(d);
   return rc;
 }
 
@@ -959,35 +986,32 @@ extern "C" int sphpc_mlp_grad(const float* d_feat, const float* d_target, int n,
   if (n <= 0 || !d_feat || !d_target || !params || !norm || !grad_out)
     return set_error(SPHPC_EINVAL, "sphpc_mlp_grad: bad arguments");
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  SPHPC_RC(set_mlp_attrs());
-  MlpDevice d;
-  TrainBufs b;
-  int rc = mlp_upload(d, params, norm, st);
+  CallNet net;
   const int grid = train_grid(n);
-  if (!rc && (cudaMalloc(&b.partial, sizeof(float) * (size_t)grid * (kMlpParams + 1)) != cudaSuccess ||
-              cudaMalloc(&b.grad, sizeof(float) * kMlpParams) != cudaSuccess ||
-              cudaMalloc(&b.loss, sizeof(float)) != cudaSuccess ||
-              cudaMalloc(&b.err, sizeof(uint32_t)) != cudaSuccess))
-    rc = set_error(SPHPC_ENOMEM, "sphpc_mlp_grad: scratch");
+  const size_t o_partial = net.part(sizeof(float) * (size_t)grid * (kMlpParams + 1));
+  int rc = net.upload(params, norm, st);
   if (!rc) {
-    cudaMemsetAsync(b.err, 0, sizeof(uint32_t), st);
-    k_mlp_grad<<<grid, kMlpTile, train_smem_bytes(), st>>>(d.params, d.norm, d.wbf, d_feat, d_target,
-                                                         n, 0, 1, 0, n, b.partial, b.err);
-    k_mlp_update<<<(kMlpParams + 256) / 256, 256, 0, st>>>(b.partial, grid, nullptr, nullptr, nullptr,
-                                                          nullptr, b.grad, b.loss, 0.f, 0.f, 0.f,
+    float* partial = net.mem.at<float>(o_partial);
+    k_mlp_grad<<<grid, kMlpTile, train_smem_bytes(), st>>>(net.d.params, net.d.norm, net.d.wbf,
+                                                           d_feat, d_target, n, 0, 1, 0, n, partial,
+                                                           net.err);
+    k_mlp_update<<<(kMlpParams + 256) / 256, 256, 0, st>>>(partial, grid, nullptr, nullptr, nullptr,
+                                                          nullptr, net.grad, net.loss, 0.f, 0.f, 0.f,
                                                           0.f, 0.f, 0.f, 0.f);
+    // loss, error word and gradient lie one after the other
+    constexpr size_t back = CallNet::kEnd - CallNet::kLoss;
+    alignas(16) unsigned char down[back];
+    cudaError_t e = cudaMemcpyAsync(down, net.loss, back, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     uint32_t h = 0;
     float ls = 0.0f;
-    cudaError_t e = cudaMemcpyAsync(grad_out, b.grad, sizeof(float) * kMlpParams,
-                                    cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&ls, b.loss, sizeof(float), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    memcpy(&ls, down, sizeof(ls));
+    memcpy(&h, down + 4, sizeof(h));
     if (e != cudaSuccess) rc = set_error(SPHPC_ECUDA, "sphpc_mlp_grad: %s", cudaGetErrorString(e));
     else if (h) rc = set_error(SPHPC_EKERNEL, "sphpc_mlp_grad: tensor-core wait gave up (0x%x)", h);
+    else memcpy(grad_out, down + (CallNet::kGrad - CallNet::kLoss), sizeof(float) * kMlpParams);
     if (!rc && loss_out) *loss_out = ls / (2.0f * (float)n);
   }
-  mlp_free(d);
   return rc;
 }
 
@@ -1078,14 +1102,14 @@ extern "C" int sphpc_mlp_dataset_stats(float* norm) {
   std::lock_guard<std::mutex> lk(g_ds_mu);
   if (g_ds.n < 2) return set_error(SPHPC_ENOTREADY, "sphpc_mlp_dataset_stats: fewer than 2 rows");
   SPHPC_RC(dataset_check_device());
-  double* acc = nullptr;
-  if (cudaMalloc(&acc, sizeof(double) * 34) != cudaSuccess)
+  CallScratch mem;
+  if (mem.take(sizeof(double) * 34, 0) != cudaSuccess)
     return set_error(SPHPC_ENOMEM, "sphpc_mlp_dataset_stats: scratch");
-  cudaMemset(acc, 0, sizeof(double) * 34);
+  double* acc = mem.at<double>(0);
+  cudaMemsetAsync(acc, 0, sizeof(double) * 34, 0);
   k_mlp_moments<<<148 * 4, 256>>>(g_ds.feat, g_ds.target, g_ds.n, acc);
   double h[34];
   const cudaError_t e = cudaMemcpy(h, acc, sizeof(h), cudaMemcpyDeviceToHost);
-  cudaFree(acc);
   if (e != cudaSuccess) return set_error(SPHPC_ECUDA, "sphpc_mlp_dataset_stats: %s", cudaGetErrorString(e));
   const double nn = (double)g_ds.n;
   for (int c = 0; c < 17; ++c) {
@@ -1125,25 +1149,19 @@ extern "C" int sphpc_mlp_train(const float* params_in, const float* norm, int st
     if (N > 0) SPHPC_RC(dataset_check_device());
   }
   if (N < 1) return set_error(SPHPC_ENOTREADY, "sphpc_mlp_train: empty training set");
-  SPHPC_RC(set_mlp_attrs());
   cudaStream_t st = 0;
-  MlpDevice d;
-  TrainBufs b;
-  int rc = mlp_upload(d, params_in, norm, st);
+  CallNet net;
   const int grid = train_grid(batch);
-  if (!rc && (cudaMalloc(&b.partial, sizeof(float) * (size_t)grid * (kMlpParams + 1)) != cudaSuccess ||
-              cudaMalloc(&b.m, sizeof(float) * kMlpParams) != cudaSuccess ||
-              cudaMalloc(&b.v, sizeof(float) * kMlpParams) != cudaSuccess ||
-              cudaMalloc(&b.loss, sizeof(float) * (size_t)(steps > 0 ? steps : 1)) != cudaSuccess ||
-              cudaMalloc(&b.err, sizeof(uint32_t)) != cudaSuccess))
-    rc = set_error(SPHPC_ENOMEM, "sphpc_mlp_train: scratch");
-  if (rc) {
-    mlp_free(d);
-    return rc;
-  }
-  cudaMemsetAsync(b.m, 0, sizeof(float) * kMlpParams, st);
-  cudaMemsetAsync(b.v, 0, sizeof(float) * kMlpParams, st);
-  cudaMemsetAsync(b.err, 0, sizeof(uint32_t), st);
+  const size_t o_partial = net.part(sizeof(float) * (size_t)grid * (kMlpParams + 1)),
+               o_m = net.part(sizeof(float) * kMlpParams), o_v = net.part(sizeof(float) * kMlpParams),
+               o_loss = net.part(sizeof(float) * (size_t)(steps > 0 ? steps : 1));
+  int rc = net.upload(params_in, norm, st);
+  if (rc) return rc;
+  const MlpDevice& d = net.d;
+  float *partial = net.mem.at<float>(o_partial), *m = net.mem.at<float>(o_m),
+        *v = net.mem.at<float>(o_v), *losses = net.mem.at<float>(o_loss);
+  cudaMemsetAsync(m, 0, sizeof(float) * kMlpParams, st);
+  cudaMemsetAsync(v, 0, sizeof(float) * kMlpParams, st);
   const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   uint64_t rng = seed;
   long long epoch = -1;
@@ -1161,15 +1179,15 @@ extern "C" int sphpc_mlp_train(const float* params_in, const float* norm, int st
       add = splitmix64(rng) % (uint64_t)N;
     }
     k_mlp_grad<<<grid, kMlpTile, train_smem_bytes(), st>>>(d.params, d.norm, d.wbf, feat, target, N,
-                                                         first % N, mul, add, batch, b.partial,
-                                                         b.err);
+                                                         first % N, mul, add, batch, partial,
+                                                         net.err);
     // cosine from lr to lr_final over the run
     const double frac = steps > 1 ? (double)(k - 1) / (double)(steps - 1) : 0.0;
     const float lr_k = (float)(lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(M_PI * frac)));
     const float bc1 = (float)(1.0 / (1.0 - std::pow((double)beta1, (double)k)));
     const float bc2 = (float)(1.0 / (1.0 - std::pow((double)beta2, (double)k)));
-    k_mlp_update<<<(kMlpParams + 256) / 256, 256, 0, st>>>(b.partial, grid, d.params, b.m, b.v,
-                                                          d.wbf, nullptr, b.loss + (k - 1), lr_k,
+    k_mlp_update<<<(kMlpParams + 256) / 256, 256, 0, st>>>(partial, grid, d.params, m, v,
+                                                          d.wbf, nullptr, losses + (k - 1), lr_k,
                                                           beta1, beta2, eps, weight_decay, bc1,
                                                           bc2);
   }
@@ -1177,13 +1195,12 @@ extern "C" int sphpc_mlp_train(const float* params_in, const float* norm, int st
   cudaError_t ce = cudaMemcpyAsync(params_out, d.params, sizeof(float) * kMlpParams,
                                    cudaMemcpyDeviceToHost, st);
   if (ce == cudaSuccess && loss_out && steps > 0)
-    ce = cudaMemcpyAsync(loss_out, b.loss, sizeof(float) * steps, cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    ce = cudaMemcpyAsync(loss_out, losses, sizeof(float) * steps, cudaMemcpyDeviceToHost, st);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h, net.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
   if (ce != cudaSuccess) rc = set_error(SPHPC_ECUDA, "sphpc_mlp_train: %s", cudaGetErrorString(ce));
   else if (h) rc = set_error(SPHPC_EKERNEL, "sphpc_mlp_train: tensor-core wait gave up (0x%x)", h);
   if (!rc && loss_out)
     for (int k = 0; k < steps; ++k) loss_out[k] /= 2.0f * (float)batch;
-  mlp_free(d);
   return rc;
 }

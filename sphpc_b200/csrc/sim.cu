@@ -16,6 +16,8 @@
 #include <utility>
 #include <vector>
 
+#include <sys/mman.h>
+
 #include "host_internal.h"
 #include "kernels.cuh"
 #include "mlp.cuh"
@@ -33,16 +35,20 @@ namespace sphpc {
 // fails with SPHPC_ENOMEM without calling cudaMalloc; -1: off.
 static std::atomic<long long> g_alloc_fail_after{-1};
 
-template <class T>
-static int dalloc(T** p, size_t n) {
-  if (n == 0) n = 1;
+static int alloc_allowed(size_t bytes) {
   long long left = g_alloc_fail_after.load();
   while (left >= 0 && !g_alloc_fail_after.compare_exchange_weak(left, left - 1)) {
   }
-  if (left == 0) {
-    *p = nullptr;
-    return set_error(SPHPC_ENOMEM, "cudaMalloc(%zu bytes): failure injected", n * sizeof(T));
-  }
+  if (left == 0)
+    return set_error(SPHPC_ENOMEM, "cudaMalloc(%zu bytes): failure injected", bytes);
+  return SPHPC_OK;
+}
+
+template <class T>
+static int dalloc(T** p, size_t n) {
+  if (n == 0) n = 1;
+  *p = nullptr;
+  SPHPC_RC(alloc_allowed(n * sizeof(T)));
   const cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
   if (e != cudaSuccess) {
     *p = nullptr;
@@ -149,7 +155,19 @@ class DeviceSim {
   std::vector<double> prof_ms;
   std::vector<int> prof_count;
 
+  // The arrays of alloc() lie in one allocation (each cudaMalloc takes about
+  // 0.4 ms, and there are 27).
+  char* arena = nullptr;
+  size_t arena_bytes = 0;
+
   ~DeviceSim() { release(); }
+
+  template <class T>
+  void drop(T*& p) {
+    const char* c = reinterpret_cast<const char*>(p);
+    if (!(arena && c >= arena && c < arena + arena_bytes)) dfree(p);
+    p = nullptr;
+  }
 
   uint32_t* gap_count() { return small; }
   uint32_t* err() { return small + 2; }
@@ -164,18 +182,18 @@ class DeviceSim {
       copy_stream = nullptr;
       copy_pending = false;
     }
-    dfree(pd); dfree(pd_alt); dfree(vel); dfree(vel_alt);
-    dfree(color); dfree(omega); dfree(dp); dfree(rho); dfree(lam);
-    dfree(color_alt); dfree(omega_alt); dfree(dp_alt); dfree(rho_alt); dfree(lam_alt);
-    dfree(ids); dfree(ids_spare); dfree(keys_by_id); dfree(loc_by_id); dfree(cellp);
-    dfree(nbr); dfree(xsa); dfree(tiles);
-    dfree(cstart); dfree(ncount); dfree(gaps); dfree(small);
-    dfree(resid); dfree(sort.keys_alt); dfree(sort.vals_alt); dfree(sort_aux); dfree(stage);
+    drop(pd); drop(pd_alt); drop(vel); drop(vel_alt);
+    drop(color); drop(omega); drop(dp); drop(rho); drop(lam);
+    drop(color_alt); drop(omega_alt); drop(dp_alt); drop(rho_alt); drop(lam_alt);
+    drop(ids); drop(ids_spare); drop(keys_by_id); drop(loc_by_id); drop(cellp);
+    drop(nbr); drop(xsa); drop(tiles);
+    drop(cstart); drop(ncount); drop(gaps); drop(small);
+    drop(resid); drop(sort.keys_alt); drop(sort.vals_alt); drop(sort_aux); drop(stage);
     mlp_release(mlp);
     for (void* h : pinned) cudaHostUnregister(h);
     pinned.clear();
-    dfree(nr); dfree(nr_alt); dfree(nr_w); dfree(lam_acc);
-    dfree(gid); dfree(owned); dfree(slab_keep); dfree(slab_counters);
+    drop(nr); drop(nr_alt); drop(nr_w); drop(lam_acc);
+    drop(gid); drop(owned); drop(slab_keep); drop(slab_counters);
     for (auto& p : pending) {
       cudaEventDestroy(p.a);
       cudaEventDestroy(p.b);
@@ -183,32 +201,59 @@ class DeviceSim {
     pending.clear();
     for (auto e : ev_pool) cudaEventDestroy(e);
     ev_pool.clear();
+    dfree(arena);
+    arena_bytes = 0;
+  }
+
+  // Every array of a particle set, to `take(pointer, count)` in a fixed order.
+  template <class F>
+  int arrays(F&& take) {
+    const size_t c = (size_t)cap;
+    SPHPC_RC(take(&pd, c)); SPHPC_RC(take(&pd_alt, c));
+    // arrays that tiles are copied from: ranges end on an even slot
+    SPHPC_RC(take(&nr, c + 2)); SPHPC_RC(take(&nr_alt, c + 2));
+    SPHPC_RC(take(&vel, c + 2)); SPHPC_RC(take(&vel_alt, c + 2));
+    SPHPC_RC(take(&color, c + 2)); SPHPC_RC(take(&omega, c)); SPHPC_RC(take(&dp, c));
+    SPHPC_RC(take(&rho, c)); SPHPC_RC(take(&lam, c));
+    SPHPC_RC(take(&ids, c)); SPHPC_RC(take(&ids_spare, c));
+    SPHPC_RC(take(&keys_by_id, c)); SPHPC_RC(take(&loc_by_id, c));
+    SPHPC_RC(take(&cellp, c)); SPHPC_RC(take(&ncount, c));
+    SPHPC_RC(take(&nbr, (size_t)kMaxNeighbors * c));
+    SPHPC_RC(take(&xsa, c + 4));  // pair blocks; the build reads four slots at a time
+    SPHPC_RC(take(&tiles, (size_t)grid_for(cap, kTileSlots)));
+    SPHPC_RC(take(&small, (size_t)8));
+    SPHPC_RC(take(&resid, (size_t)16));
+    SPHPC_RC(take(&sort.keys_alt, c));
+    SPHPC_RC(take(&sort.vals_alt, c));
+    return take(&sort_aux, sort_aux_words(cap));
   }
 
   int alloc(int n_, int cap_) {
     n = n_;
     cap = cap_ > n_ ? cap_ : n_;
     const int c = cap;
-    SPHPC_RC(dalloc(&pd, c)); SPHPC_RC(dalloc(&pd_alt, c));
-    // arrays that tiles are copied from: ranges end on an even slot
-    SPHPC_RC(dalloc(&nr, (size_t)c + 2)); SPHPC_RC(dalloc(&nr_alt, (size_t)c + 2));
-    SPHPC_RC(dalloc(&vel, (size_t)c + 2)); SPHPC_RC(dalloc(&vel_alt, (size_t)c + 2));
-    SPHPC_RC(dalloc(&color, (size_t)c + 2)); SPHPC_RC(dalloc(&omega, c)); SPHPC_RC(dalloc(&dp, c));
-    SPHPC_RC(dalloc(&rho, c)); SPHPC_RC(dalloc(&lam, c));
-    SPHPC_RC(dalloc(&ids, c)); SPHPC_RC(dalloc(&ids_spare, c));
-    SPHPC_RC(dalloc(&keys_by_id, c)); SPHPC_RC(dalloc(&loc_by_id, c));
-    SPHPC_RC(dalloc(&cellp, c)); SPHPC_RC(dalloc(&ncount, c));
-    SPHPC_RC(dalloc(&nbr, (size_t)kMaxNeighbors * c));
-    SPHPC_RC(dalloc(&xsa, (size_t)c + 4));  // pair blocks; the build reads four slots at a time
-    SPHPC_RC(dalloc(&tiles, (size_t)grid_for(c, kTileSlots)));
-    SPHPC_CK(cudaMemsetAsync(ncount, 0, c, stream));
-    SPHPC_RC(dalloc(&small, 8));
-    SPHPC_RC(dalloc(&resid, 16));
-    SPHPC_RC(dalloc(&sort.keys_alt, c));
-    SPHPC_RC(dalloc(&sort.vals_alt, c));
-    const size_t aux = sort_aux_words(c);
-    SPHPC_RC(dalloc(&sort_aux, aux));
+    auto padded = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    size_t total = 0;
+    SPHPC_RC(arrays([&](auto p, size_t count) {
+      total += padded(count * sizeof(**p));
+      return alloc_allowed(count * sizeof(**p));
+    }));
+    const cudaError_t e = cudaMalloc(&arena, total);
+    if (e != cudaSuccess) {
+      arena = nullptr;
+      cudaGetLastError();
+      return set_error(SPHPC_ENOMEM, "cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
+    }
+    arena_bytes = total;
+    size_t at = 0;
+    SPHPC_RC(arrays([&](auto p, size_t count) {
+      *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(arena + at);
+      at += padded(count * sizeof(**p));
+      return SPHPC_OK;
+    }));
+    const size_t aux = sort_aux_words(cap);
     sort_layout(sort, sort_aux);
+    SPHPC_CK(cudaMemsetAsync(ncount, 0, c, stream));
     SPHPC_CK(cudaMemsetAsync(small, 0, 8 * sizeof(uint32_t), stream));
     SPHPC_CK(cudaMemsetAsync(sort_aux, 0, aux * sizeof(uint32_t), stream));
     SPHPC_CK(cudaMemsetAsync(pd, 0, sizeof(PD) * c, stream));
@@ -982,7 +1027,29 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-static int enter_data(Particles* particles, const Params* params, DeviceSim** out) {
+// Fields that AllocInitParticles lays on whole pages: position, velocity and
+// density (a frame's and a state's), from this size on.
+constexpr int kStateFields = 7;
+constexpr size_t kLockBytes = (size_t)2 << 20;
+
+// A zeroed host array of n doubles, for free().  From 2 MB on it starts on a 2 MB
+// boundary and fills whole 2 MB pages, which are asked of the kernel as huge
+// pages: touching and page-locking them then takes a half and a quarter of the
+// time of 4 KB pages.
+static double* host_array(size_t n) {
+  const size_t bytes = n * sizeof(double), page = (size_t)2 << 20;
+  if (bytes < kLockBytes) return (double*)calloc(n, sizeof(double));
+  const size_t whole = (bytes + page - 1) & ~(page - 1);
+  void* p = aligned_alloc(page, whole);
+  if (!p) return nullptr;
+  madvise(p, whole, MADV_HUGEPAGE);
+  memset(p, 0, bytes);
+  return (double*)p;
+}
+
+// whole_pages: the host arrays of the first kStateFields fields come from
+// host_array.
+static int enter_data(Particles* particles, const Params* params, bool whole_pages) {
   if (!particles || !params) return set_error(SPHPC_EINVAL, "sphpc_enter_data: null argument");
   if (particles->local_count <= 0 || !particles->x || !particles->y || !particles->z)
     return set_error(SPHPC_EINVAL, "sphpc_enter_data: no particles");
@@ -1001,22 +1068,27 @@ static int enter_data(Particles* particles, const Params* params, DeviceSim** ou
   s->mass = particles->rest_mass;
   int rc = s->alloc(particles->local_count, particles->max_local);
   if (!rc) {
-    // Page-lock the large host arrays in place: the reference's calloc'd
-    // arrays stay the caller's, only their transfers get faster.  Arrays
-    // below 64 MB may share pages with other allocations and are left
-    // pageable, as is any array the driver refuses to register.
+    // Page-lock host arrays in place, so that their transfers run at the link's
+    // speed (15 MB to the host: 762 us pageable, 286 us locked).  Arrays of 64 MB
+    // and more: all of them, the reference's calloc'd ones too.  Smaller ones may
+    // share pages with other allocations and are left pageable, except those
+    // that AllocInitParticles laid on whole pages: the fields of a frame and of a
+    // state, from kLockBytes on (locking costs 0.35 ms an array and more, for 97k
+    // particles 5 ms a set against 0.3 ms a read-back of the state).  An array that the driver refuses stays
+    // pageable.
     const size_t bytes = sizeof(double) * (size_t)particles->max_local;
-    if (bytes >= ((size_t)64 << 20)) {
-      double* fields[20] = {particles->x_star, particles->y_star, particles->z_star, particles->x,
-                            particles->y, particles->z, particles->v_x, particles->v_y,
-                            particles->v_z, particles->dp_x, particles->dp_y, particles->dp_z,
-                            particles->w_x, particles->w_y, particles->w_z, particles->color_x,
-                            particles->color_y, particles->color_z, particles->density,
+    if (bytes >= ((size_t)64 << 20) || (whole_pages && bytes >= kLockBytes)) {
+      double* fields[20] = {particles->x, particles->y, particles->z, particles->v_x,
+                            particles->v_y, particles->v_z, particles->density, particles->x_star,
+                            particles->y_star, particles->z_star, particles->dp_x, particles->dp_y,
+                            particles->dp_z, particles->w_x, particles->w_y, particles->w_z,
+                            particles->color_x, particles->color_y, particles->color_z,
                             particles->lambda};
-      for (double* f : fields) {
-        if (!f) continue;
-        if (cudaHostRegister(f, bytes, cudaHostRegisterDefault) == cudaSuccess)
-          s->pinned.push_back(f);
+      const int count = bytes >= ((size_t)64 << 20) ? 20 : kStateFields;
+      for (int k = 0; k < count; ++k) {
+        if (!fields[k]) continue;
+        if (cudaHostRegister(fields[k], bytes, cudaHostRegisterDefault) == cudaSuccess)
+          s->pinned.push_back(fields[k]);
         else
           cudaGetLastError();
       }
@@ -1036,7 +1108,6 @@ static int enter_data(Particles* particles, const Params* params, DeviceSim** ou
     delete s;
     return rc;
   }
-  if (out) *out = s;
   return SPHPC_OK;
 }
 
@@ -1080,7 +1151,7 @@ extern "C" {
 
 int sphpc_enter_data(struct Particles* particles, const struct Params* params) {
   clear_error();
-  return enter_data(particles, params, nullptr);
+  return enter_data(particles, params, false);
 }
 
 int sphpc_exit_data(struct Particles* particles) {
@@ -1226,8 +1297,12 @@ int AllocInitParticles(struct Particles* particles, struct Params* params,
                           &particles->dp_z, &particles->w_x, &particles->w_y, &particles->w_z,
                           &particles->color_x, &particles->color_y, &particles->color_z,
                           &particles->density, &particles->lambda};
+  const bool large = n * sizeof(double) >= ((size_t)64 << 20);
   for (auto f : dfields) {
-    *f = (double*)calloc(n, sizeof(double));
+    const bool state = f == &particles->x || f == &particles->y || f == &particles->z ||
+                       f == &particles->v_x || f == &particles->v_y || f == &particles->v_z ||
+                       f == &particles->density;
+    *f = large || state ? host_array(n) : (double*)calloc(n, sizeof(double));
     if (!*f) return set_error(SPHPC_ENOMEM, "AllocInitParticles: calloc of %zu doubles", n);
   }
   particles->id = (int*)calloc(n, sizeof(int));
@@ -1258,7 +1333,7 @@ int AllocInitParticles(struct Particles* particles, struct Params* params,
   }
   particles->halo_count_left = 0;
   particles->halo_count_right = 0;
-  return enter_data(particles, params, nullptr);
+  return enter_data(particles, params, true);
 }
 
 int FinalizeParticles(struct Particles* particles) {

@@ -52,13 +52,14 @@ using CtxGetCurrentFn = int (*)(void**);
 using CtxGetIdFn = int (*)(void*, unsigned long long*);
 CtxGetCurrentFn g_ctx_get_current = nullptr;
 CtxGetIdFn g_ctx_get_id = nullptr;
-bool g_ctx_fns_tried = false;
+std::once_flag g_ctx_fns_once;
 
-// Unique id of the current context; false when the driver cannot say (then
-// the address is looked up again on every call).
-bool current_ctx_id(unsigned long long* id) {
-  if (!g_ctx_fns_tried) {
-    g_ctx_fns_tried = true;
+}  // namespace
+
+// (The callers here look the address up again on every call where this is
+// false.)
+bool current_context_id(unsigned long long* id) {
+  std::call_once(g_ctx_fns_once, [] {
     void* f = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
@@ -69,12 +70,14 @@ bool current_ctx_id(unsigned long long* id) {
         q == cudaDriverEntryPointSuccess)
       g_ctx_get_id = reinterpret_cast<CtxGetIdFn>(f);
     cudaGetLastError();
-  }
+  });
   if (!g_ctx_get_current || !g_ctx_get_id) return false;
   void* ctx = nullptr;
   if (g_ctx_get_current(&ctx) != 0 || !ctx) return false;
   return g_ctx_get_id(ctx, id) == 0;
 }
+
+namespace {
 
 // Device address of g_noalloc_scratch on the current device.  In host code
 // the array's name is only a host-side stand-in, so the address comes from
@@ -92,7 +95,7 @@ int scratch_address(uint32_t** out) {
   // or right after a reset) counts as unknown: cudaGetSymbolAddress below
   // makes the primary context current, and the next call records its id
   unsigned long long id = 0;
-  const bool known = current_ctx_id(&id);
+  const bool known = current_context_id(&id);
   if (!slot.ptr || !known || !slot.ctx_known || slot.ctx_id != id) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "host_internal.h"
+#include "scratch.cuh"
 
 namespace sphpc {
 namespace {
@@ -102,13 +103,15 @@ extern "C" int sphpc_particle_surface(const double* xyz, int np, double radius, 
   const float band = half_width * voxel + r;
   if ((double)band * kFixScale > 2.0e9)
     return set_error(SPHPC_EINVAL, "sphpc_particle_surface: radius too large for the grid units");
-  double* d_xyz = nullptr;
-  int* d_fix = nullptr;
-  float *d_a = nullptr, *d_b = nullptr;
-  cudaError_t e = cudaMalloc(&d_xyz, sizeof(double) * 3 * (size_t)np);
-  if (e == cudaSuccess) e = cudaMalloc(&d_fix, sizeof(int) * (size_t)n);
-  if (e == cudaSuccess) e = cudaMalloc(&d_a, sizeof(float) * (size_t)n);
-  if (e == cudaSuccess) e = cudaMalloc(&d_b, sizeof(float) * (size_t)n);
+  ScratchLayout lay;
+  const size_t o_xyz = lay.part(sizeof(double) * 3 * (size_t)np),
+               o_fix = lay.part(sizeof(int) * (size_t)n), o_a = lay.part(sizeof(float) * (size_t)n),
+               o_b = lay.part(sizeof(float) * (size_t)n);
+  CallScratch mem;
+  cudaError_t e = mem.take(lay.bytes(), 0);
+  double* d_xyz = mem.at<double>(o_xyz);
+  int* d_fix = mem.at<int>(o_fix);
+  float *d_a = mem.at<float>(o_a), *d_b = mem.at<float>(o_b);
   if (e == cudaSuccess)
     e = cudaMemcpy(d_xyz, xyz, sizeof(double) * 3 * (size_t)np, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
@@ -130,10 +133,6 @@ extern "C" int sphpc_particle_surface(const double* xyz, int np, double radius, 
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(phi, d_a, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost);
-  cudaFree(d_xyz);
-  cudaFree(d_fix);
-  cudaFree(d_a);
-  cudaFree(d_b);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(SPHPC_ECUDA, "sphpc_particle_surface: %s", cudaGetErrorString(e));
