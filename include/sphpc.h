@@ -153,11 +153,15 @@ int sphpc_get_cell_data(const struct Particles *particles, unsigned int *hash_va
 /* No counterpart in the reference (whose FillNeighbors tests every pair in
  * FP64, neighbors.c:278-285).  1 if the neighbour build's FP32 candidate
  * pre-test decides r^2 < h^2 exactly as that FP64 test does for
- * coordinates of magnitude up to max_coord (it leaves pairs within
- * +-2^-10 h^2 of h^2 to the FP64 test); 0 otherwise, in which case the
+ * coordinates of magnitude up to max_coord (it leaves pairs within a band
+ * about h^2 to the FP64 test); 0 otherwise, in which case the
  * build sends every candidate to the FP64 test.  The build applies it with
  * max_coord = h * max(hash_size_x, hash_size_y, hash_size_z). */
 int sphpc_neighbor_pretest_fp32_safe(double max_coord, double h);
+
+/* The half width of that band: how far FP32 rounding can move r^2 near h^2
+ * at max_coord, at most 2^-10 h^2; infinite where the pre-test is not safe. */
+double sphpc_neighbor_pretest_band(double max_coord, double h);
 
 /* ---------------- slab decomposition along x (communication.c) ---------------- */
 

@@ -253,10 +253,10 @@ __device__ __forceinline__ bool axis_regular(double x, double h, int c, int nmax
 
 // r^2 < h^2 exactly as neighbors.c:278-285 evaluates it on the canonical
 // double positions of slots p and j.  The FP32 absolute positions decide every
-// pair whose r^2 lies outside the band [P.bld_h2lo, P.bld_h2hi] = h^2 (1 -+
-// 2^-10); this test decides the rest.  The host opens the band to every pair
-// when FP32 rounding of the grid's largest coordinate could move r^2 by that
-// much (sphpc_neighbor_pretest_fp32_safe: beyond about 2^12 h).
+// pair whose r^2 lies outside the band [P.bld_h2lo, P.bld_h2hi] about h^2; this
+// test decides the rest.  The band is as wide as FP32 rounding of the grid's
+// largest coordinate can move r^2 (sphpc_neighbor_pretest_band: 2^-14 h^2 for 128
+// cells an axis), and open to every pair beyond about 2^12 h.
 __device__ __forceinline__ bool exact_neighbor(const DevParams& P, const PD* __restrict__ pd,
                                                int p, int j) {
   float4 xp, dp, xq, dq;
@@ -310,35 +310,37 @@ __device__ __forceinline__ int walk_27_cells(const DevParams& P, const NbrView& 
 
 // ---------------------------------------------------------------------------
 // Neighbour build (FillNeighbors, neighbors.c:217-298): one thread per
-// particle walks its 9 (dz, dy) slot rows in the reference's order (rows of
+// particle tests its 9 (dz, dy) slot rows in the reference's order (rows of
 // cells cx-1..cx+1 are contiguous slot ranges, cells in dx order, particles
-// in ascending original index), appending every candidate without branches
-// to its own column of a shared-memory staging area -- store the entry,
-// advance the count on a hit -- and writes its bucket out at the end as
-// 16-byte blocks (for each block index, a warp's 32 consecutive slots are
-// four whole 128-byte lines), the last block's entries past the count set to
-// the particle itself.
+// in ascending original index), four candidates at a time without branches,
+// each hit one bit shifted into a word of 32 candidates.  The words that hold a
+// hit go to the thread's column in shared memory, and the list is written from
+// them at the end as 16-byte blocks (for each block index, a warp's 32
+// consecutive slots are four whole 128-byte lines), the last block's entries
+// past the count set to the particle itself.
 //
 // The candidates of a block of kTileSlots slots come from its tile of FP32
 // positions in shared memory (TileInfo; nine bulk copies), pairs of slots as
-// the 64-bit operands of the packed FP32x2 arithmetic of sm_100, and a staged
-// entry is the candidate's byte offset in the record tile, which is also the
-// list's entry.  A block whose tile does not fit loads the pairs from global
-// memory and stages (row << 12) | offset in the row, with the row starts in
-// shared memory.  A particle with a row of more than 4095 candidates takes the
-// verbatim 27-cell walk.
+// the 64-bit operands of the packed FP32x2 arithmetic of sm_100, and the list's
+// entries are byte offsets in the record tile.  A block whose tile does not fit
+// loads the pairs from global memory and its list holds slots.
 //
-// Bounds: instruction issue (71%) and the shared-memory pipe (74%) together,
-// at five blocks per SM.  16.7M particles: 4024 us with every candidate pair
-// loaded per lane from global memory (the L1 data pipe at 88%), 3394 us so.
-// Tried for the same work and slower: the candidates of a cell held by a
-// warp's lanes, its particles broadcast to them and the hits taken from
-// ballots (240 warp instructions a particle against 136; 4.2M particles: 1462
-// us against 848).
+// Bound: instruction issue (79% at 41% of the warps), 118 warp instructions a
+// particle.  4.2M particles: 1005 us with candidate pairs loaded per lane from
+// global memory and every candidate stored and counted on a hit; 854 us so from
+// tiles, the shared-memory pipe then as busy as the issue (74%, half of it bank
+// conflicts: the lanes of a warp are in four cells whose rows start a cell's
+// eight records, one turn of the banks, apart); 739 us with hit words; 663 us
+// with the lanes of odd cells half a turn of the banks ahead (conflicts 17M ->
+// 4M a launch of 1M particles) and the band as narrow as the grid allows; 618 us
+// with the words read back without a test a hit.  Tried for the same work and
+// slower: the candidates of a cell held by a warp's lanes, its particles
+// broadcast to them and the hits taken from ballots (1462 us).
+//
+// kWords: rows at rest density take one word; with ten a column seven blocks
+// fit an SM.  A particle with more writes whole blocks of its list ahead.
 // ---------------------------------------------------------------------------
-constexpr int kRowBits = 12;
-constexpr int kRowMax = (1 << kRowBits) - 1;
-constexpr int kStageRows = kMaxNeighbors + 4;  // four candidates are appended at a time
+constexpr int kWords = 10;
 
 // Whether the neighbour cells of a particle with FP32 position x in cell c of
 // an axis are c-1, c, c+1 (axis_regular) for certain: x / h lies at least
@@ -349,6 +351,12 @@ __device__ __forceinline__ bool axis_inside(float x, float inv_h, int c) {
   return f > m && f < 1.0f - m;
 }
 
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float m;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+
 struct BuildRow {
   const DevParams& P;
   const PD* __restrict__ pd;
@@ -356,19 +364,20 @@ struct BuildRow {
   int p;
 };
 
-// Tests and appends candidates j .. j+3 (j even) of the range [lo, hi): with
-// MASK those outside it, and `skip`, are left out.  `slot` - j is the slot of
-// index 0.  s = r^2 - h^2 by fused multiply-adds from -h^2: its sign decides,
-// and the exact FP64 test where |s| lies in the band (the three roundings of
-// s stay within the bound that the band was sized for: near the band every
-// partial sum is at most h^2).
-template <bool TILE, bool MASK>
-__device__ __forceinline__ void build_four(const BuildRow& c, const float4* __restrict__ src, int j,
-                                           int lo, int hi, int skip, int dslot, uint32_t entry,
-                                           uint16_t* __restrict__ stg, int& cnt) {
+// Tests the candidates of `group` = src + j, j even, and the three after it and shifts their hits into `word`, the
+// first one highest.  Candidate j is slot j + dslot.
+// s = r^2 - h^2 by fused multiply-adds from -h^2: its sign decides, and the
+// exact FP64 test where |s| lies in the band (the three roundings of s stay
+// within the bound that the band was sized for: near the band every partial
+// sum is at most h^2).  Candidates outside [lo, hi) may be any bits: they are
+// tested by sign alone, and the caller drops their hits.
+template <bool TILE>
+__device__ __forceinline__ uint32_t build_four(const BuildRow& c, const float4* __restrict__ src,
+                                               const float4* __restrict__ group, int lo, int hi,
+                                               int dslot, uint32_t word) {
   uint64_t x0, y0, z0, x1, y1, z1;
   if (TILE) {
-    const ulonglong2* t = reinterpret_cast<const ulonglong2*>(src + j);
+    const ulonglong2* t = reinterpret_cast<const ulonglong2*>(group);
     const ulonglong2 a = t[0], b = t[2];
     x0 = a.x;
     y0 = a.y;
@@ -377,8 +386,8 @@ __device__ __forceinline__ void build_four(const BuildRow& c, const float4* __re
     z0 = *reinterpret_cast<const uint64_t*>(t + 1);
     z1 = *reinterpret_cast<const uint64_t*>(t + 3);
   } else {
-    ld_pair(src, j, x0, y0, z0);
-    ld_pair(src, j + 2, x1, y1, z1);
+    ld_pair(group, 0, x0, y0, z0);
+    ld_pair(group, 2, x1, y1, z1);
   }
   uint64_t d = f2_sub(c.pxx, x0);
   uint64_t s0 = f2_fma(d, d, c.mh2);
@@ -394,89 +403,154 @@ __device__ __forceinline__ void build_four(const BuildRow& c, const float4* __re
   s1 = f2_fma(d, d, s1);
   float s[4] = {f2_lo(s0), f2_hi(s0), f2_lo(s1), f2_hi(s1)};
   const float band = c.P.bld_band;
-  auto inside = [&](int u) {
-    return (unsigned)(j + u - lo) < (unsigned)(hi - lo) && j + u != skip;
-  };
-  if (MASK) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) s[u] = inside(u) ? s[u] : 3.0e38f;
-  }
-  const float m = fminf(fminf(fabsf(s[0]), fabsf(s[1])), fminf(fabsf(s[2]), fabsf(s[3])));
-  if (m <= band) {
+  if (fminf(min3_abs(s[0], s[1], s[2]), fabsf(s[3])) <= band) {
+    const int j = (int)(group - src);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (fabsf(s[u]) <= band && (!MASK || inside(u)))
+      if (fabsf(s[u]) <= band && j + u >= lo && j + u < hi)
         s[u] = exact_neighbor(c.P, c.pd, c.p, j + u + dslot) ? -1.0f : 1.0f;
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    stg[cnt * kTileSlots] = (uint16_t)(entry + (TILE ? 16 * u : u));
-    cnt += s[u] < 0.0f ? 1 : 0;
-  }
+  for (int u = 0; u < 4; ++u) word = __funnelshift_l(__float_as_uint(s[u]), word, 1);
+  return word;
 }
 
-// Appends the candidates [lo, hi) of one row except `skip` (< 0: none).
-template <bool TILE, bool SKIP>
+// The hits of one particle between the tests and its list: words of 32
+// consecutive candidates that hold a hit, in list order, in the thread's columns
+// (stride kTileSlots) of `mask` and `base`; base is the list entry of the word's
+// lowest bit, and entries fall by 1 << SHIFT a bit upwards.
+template <class B, int SHIFT>
+struct Hits {
+  uint32_t* mask;
+  B* base;
+  int words = 0;      // stored
+  int found = 0;      // hits so far, at most kMaxNeighbors
+  int written = 0;    // entries in the list
+
+  // Writes the list's blocks while more than `keep` hits are not written.
+  __device__ __forceinline__ void write(uint4*& out, int n, int keep) {
+    constexpr int kPer = sizeof(B) == 2 ? 8 : 4;
+    int next = 0;
+    uint32_t m = 0, e0 = 0;
+    auto take = [&]() -> uint32_t {
+      if (m == 0) {
+        m = mask[next * kTileSlots];
+        e0 = (uint32_t)base[next * kTileSlots];
+        next = min(next + 1, words);
+      }
+      const int f = 31 - __clz((int)m);
+      m &= ~(1u << f);
+      return e0 - ((uint32_t)f << SHIFT);
+    };
+#pragma unroll 1
+    for (; found - written > keep; out += n, written += kPer) {
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        w[u] = take();
+        if (kPer == 8) w[u] |= take() << 16;
+      }
+      *out = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (keep == 0) return;
+    // what is left moves to the front
+    int k = 0;
+    if (m != 0) {
+      mask[0] = m;
+      base[0] = (B)e0;
+      k = 1;
+    }
+    for (; next < words; ++next, ++k) {
+      mask[k * kTileSlots] = mask[next * kTileSlots];
+      base[k * kTileSlots] = base[next * kTileSlots];
+    }
+    words = k;
+  }
+
+  __device__ __forceinline__ void add(uint32_t word, uint32_t entry, uint4*& out, int n) {
+    if (word == 0) return;
+    // (at most seven hits, in as many words, stay)
+    if (words == kWords) write(out, n, 7);
+    found += __popc(word);
+    for (; found > kMaxNeighbors; --found) word &= word - 1;
+    mask[words * kTileSlots] = word;
+    base[words * kTileSlots] = (B)entry;
+    ++words;
+  }
+
+  // The rest of the list, the last block filled up with entry `self`: a word of
+  // one hit that is read over and over.
+  __device__ __forceinline__ void finish(uint32_t self, uint4*& out, int n) {
+    mask[words * kTileSlots] = 1u;
+    base[words * kTileSlots] = (B)self;
+    write(out, n, 0);
+  }
+};
+
+// The hits among candidates [lo, hi) of one row except `skip` (< 0: none).
+template <bool TILE, class H>
 __device__ __forceinline__ void build_range(const BuildRow& c, const float4* __restrict__ src,
-                                            int lo, int hi, int skip, int dslot, uint32_t tag,
-                                            uint16_t* __restrict__ stg, int& cnt) {
-  if (lo >= hi || cnt >= kMaxNeighbors) return;
-  // (the first group may start one slot before lo: its offset -1 is not taken)
-  auto entry = [&](int j) {
-    return TILE ? (uint32_t)j << 4 : (tag << kRowBits) + (uint32_t)(j - lo);
-  };
-  int j = lo & ~1;
-  build_four<TILE, true>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
-  j += 4;
-  for (; j + 4 <= hi && cnt < kMaxNeighbors; j += 4)
-    build_four<TILE, SKIP>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
-  if (j < hi && cnt < kMaxNeighbors)
-    build_four<TILE, true>(c, src, j, lo, hi, skip, dslot, entry(j), stg, cnt);
+                                            int lo, int hi, int skip, int dslot, int odd,
+                                            H& hits, uint4*& out, int n) {
+  for (int w = lo & ~1; w < hi && hits.found < kMaxNeighbors; w += 32) {
+    const int end = min(w + 32, hi), bits = (end - w + 3) & ~3;
+    // Lanes of adjacent cells read different halves of the 128 bytes that the
+    // banks hold of a tile's pairs: those of the wrong parity start with the
+    // second group of four and take the first one last.
+    const bool turn = TILE && (((w >> 2) ^ odd) & 1) != 0;
+    uint32_t word = 0;
+    const float4* g = src + w + (turn ? 4 : 0);
+    const float4* const g1 = g + bits - 4;
+#pragma unroll 1
+    for (; g != g1; g += 4) word = build_four<TILE>(c, src, g, lo, hi, dslot, word);
+    word = build_four<TILE>(c, src, turn ? src + w : g, lo, hi, dslot, word);
+    word <<= 32 - bits;
+    if (turn) {
+      const uint32_t first = word & (15u << (32 - bits));
+      word = ((word ^ first) >> 4) | (first << (bits - 4));
+    }
+    if (w < lo) word &= 0x7fffffffu;
+    word &= 0xffffffffu << (32 - (end - w));
+    if ((unsigned)(skip - w) < 32u) word &= ~(0x80000000u >> (skip - w));
+    hits.add(word, (uint32_t)(w + 31) << (TILE ? 4 : 0), out, n);
+  }
 }
 
 // The nine rows of particle p, tile: src is the tile and off[r] = o[r] - s[r]
-// takes slots to tile records; else src is xsa and rowb receives the row
-// starts (stride kTileSlots).  Returns the staged count, at most
-// kMaxNeighbors, or -1 for a row beyond kRowMax (without a tile).
-template <bool TILE>
-__device__ __forceinline__ int build_rows(const BuildRow& c, const NbrView& V, uint32_t cell,
-                                          const float4* __restrict__ src, const int* off,
-                                          int* rowb, uint16_t* __restrict__ stg) {
+// takes slots to tile records; else src is xsa.
+template <bool TILE, class H>
+__device__ __forceinline__ void build_rows(const BuildRow& c, const NbrView& V, uint32_t cell,
+                                           const float4* __restrict__ src, const int* off, H& hits,
+                                           uint4*& out) {
   const DevParams& P = c.P;
   int cx, cy, cz;
   unpack_cell(V, cell, cx, cy, cz);
-  const int xlo = cx - (cx > 0), xhi = cx + (cx < P.nx - 1) + 1;
+  // rows of the grid among the nine
+  const uint32_t ys = (cy > 0 ? 1u : 0u) | 2u | (cy < P.ny - 1 ? 4u : 0u);
+  const uint32_t rows = (cz > 0 ? ys : 0u) | ys << 3 | (cz < P.nz - 1 ? ys << 6 : 0u);
+  const uint32_t* first = V.cstart + (cx - (cx > 0));
+  const int width = (cx > 0) + 1 + (cx < P.nx - 1);
+  uint32_t key = (uint32_t)cz * P.nxny + (uint32_t)cy * (uint32_t)P.nx - P.nxny - (uint32_t)P.nx;
   auto bounds = [&](int r, int& b, int& e) {
-    const int z = cz + r / 3 - 1, y = cy + r % 3 - 1;
     b = e = 0;
-    if (r < 9 && (unsigned)z < (unsigned)P.nz && (unsigned)y < (unsigned)P.ny) {
-      const uint32_t rk = (uint32_t)z * P.nxny + (uint32_t)y * (uint32_t)P.nx;
-      b = (int)__ldg(V.cstart + rk + xlo);
-      e = (int)__ldg(V.cstart + rk + xhi);
+    if (rows >> r & 1u) {
+      b = (int)__ldg(first + key);
+      e = (int)__ldg(first + key + width);
     }
+    key += (uint32_t)P.nx;
+    if (r % 3 == 2) key += P.nxny - 3u * (uint32_t)P.nx;
   };
-  if (!TILE) {
-    for (int r = 0; r < 9; ++r) {
-      int b, e;
-      bounds(r, b, e);
-      if (e - b > kRowMax) return -1;
-    }
-  }
-  int cnt = 0, b, e;
+  int b, e;
   bounds(0, b, e);
+#pragma unroll 1
   for (int r = 0; r < 9; ++r) {
     int bn, en;
     bounds(r + 1, bn, en);  // the next row's, ahead of this row's tests
     const int o = TILE ? off[r] : 0;
-    if (!TILE) rowb[r * kTileSlots] = b;
-    if (r == 4)
-      build_range<TILE, true>(c, src, b + o, e + o, c.p + o, -o, (uint32_t)r, stg, cnt);
-    else
-      build_range<TILE, false>(c, src, b + o, e + o, -1, -o, (uint32_t)r, stg, cnt);
+    build_range<TILE>(c, src, b + o, e + o, r == 4 ? c.p + o : -1, -o, cx, hits, out, V.n);
     b = bn;
     e = en;
   }
-  return min(cnt, kMaxNeighbors);
 }
 
 // The nine ranges of the block's tile (TileInfo): computed by lanes 0..8 of
@@ -512,22 +586,17 @@ __device__ __forceinline__ void tile_ranges(const DevParams& P, const NbrView& V
   if (r == 8) t.total = o;
 }
 
-// Staging column of a thread: halfwords of warps 2k and 2k + 1 share a 32-bit
-// word, so a warp's 32 columns lie in 32 banks whatever their counts.
-__device__ __forceinline__ int stage_column() {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  return ((warp >> 1) * 32 + lane) * 2 + (warp & 1);
-}
-
-// Five blocks of 128 threads per SM with their tiles (40 KB).
-__global__ void __launch_bounds__(kTileSlots, 5)
+// Seven blocks of 128 threads per SM with their tiles (32 KB).
+__global__ void __launch_bounds__(kTileSlots, 7)
     k_build(const DevParams P, const NbrView V, const PD* __restrict__ pd,
             const float4* __restrict__ xsa, const uint32_t* __restrict__ cellp,
             uint32_t* __restrict__ nbr, uint8_t* __restrict__ ncount, TileInfo* __restrict__ tiles) {
   // the tile (its last group of four may read three records past it), or the
-  // row starts of a block without one
+  // bases of the hit words of a block without one
   __shared__ __align__(128) float4 s_tile[kTileCap + 4];
-  __shared__ uint16_t s_stage[kStageRows * kTileSlots];
+  __shared__ uint32_t s_mask[(kWords + 1) * kTileSlots];
+  __shared__ uint16_t s_base[(kWords + 1) * kTileSlots];
+  static_assert(sizeof(int) * (kWords + 1) * kTileSlots <= sizeof(s_tile), "bases fit in the tile");
   __shared__ TileInfo s_info;
   __shared__ int s_off[9];
   __shared__ __align__(8) uint64_t s_mbar;
@@ -582,40 +651,21 @@ __global__ void __launch_bounds__(kTileSlots, 5)
     mbar_wait0(&s_mbar);
   }
   if (!own) return;
-  uint16_t* stg = s_stage + stage_column();
   const BuildRow c{P, pd, f2_dup(xf.x), f2_dup(xf.y), f2_dup(xf.z), f2_dup(-P.h2), p};
   uint4* out = reinterpret_cast<uint4*>(nbr) + p;
   int count;
   if (tiled) {
-    count = build_rows<true>(c, V, cell, s_tile, s_off, nullptr, stg);
-    const uint32_t self = (uint32_t)(p + s_off[4]) << 4;
-#pragma unroll 1
-    for (int t0 = 0; t0 < count; t0 += 8, out += P.n) {
-      uint32_t w[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = t0 + 2 * u;
-        const uint32_t a = t < count ? stg[t * kTileSlots] : self;
-        const uint32_t b = t + 1 < count ? stg[(t + 1) * kTileSlots] : self;
-        w[u] = a | (b << 16);
-      }
-      *out = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    Hits<uint16_t, 4> hits{s_mask + threadIdx.x, s_base + threadIdx.x};
+    build_rows<true>(c, V, cell, s_tile, s_off, hits, out);
+    hits.finish((uint32_t)(p + s_off[4]) << 4, out, P.n);
+    count = hits.found;
+  } else if (regular) {
+    Hits<int, 0> hits{s_mask + threadIdx.x, reinterpret_cast<int*>(s_tile) + threadIdx.x};
+    build_rows<false>(c, V, cell, xsa, nullptr, hits, out);
+    hits.finish((uint32_t)p, out, P.n);
+    count = hits.found;
   } else {
-    int* rowb = reinterpret_cast<int*>(s_tile) + threadIdx.x;
-    count = regular ? build_rows<false>(c, V, cell, xsa, nullptr, rowb, stg) : -1;
-    if (count < 0) {
-      count = walk_27_cells(P, V, pd, xsa, p, nbr);
-    } else {
-      auto entry = [&](int t) {
-        if (t >= count) return (uint32_t)p;
-        const uint32_t en = stg[t * kTileSlots];
-        return (uint32_t)(rowb[(en >> kRowBits) * kTileSlots] + (int)(en & kRowMax));
-      };
-#pragma unroll 1
-      for (int t0 = 0; t0 < count; t0 += 4, out += P.n)
-        *out = make_uint4(entry(t0), entry(t0 + 1), entry(t0 + 2), entry(t0 + 3));
-    }
+    count = walk_27_cells(P, V, pd, xsa, p, nbr);
   }
   ncount[p] = (uint8_t)count;
 }

@@ -485,15 +485,10 @@ DevParams DeviceSim::params(const Params& prm, const AABB* b, const Obstacle* ob
   {
     // coordinates that hash inside the grid lie below max(nx, ny, nz) h
     const int nmax = std::max(nx, std::max(ny, nz));
-    if (sphpc_neighbor_pretest_fp32_safe((double)nmax * h, h)) {
-      P.bld_h2lo = (float)(h * h) * (1.0f - 1.0f / 1024.0f);
-      P.bld_h2hi = (float)(h * h) * (1.0f + 1.0f / 1024.0f);
-      P.bld_band = (float)(h * h) * (1.0f / 1024.0f);
-    } else {
-      P.bld_h2lo = -1.0f;
-      P.bld_h2hi = INFINITY;
-      P.bld_band = INFINITY;
-    }
+    const double band = sphpc_neighbor_pretest_band((double)nmax * h, h);
+    P.bld_band = std::isfinite(band) ? std::nextafterf((float)band, INFINITY) : INFINITY;
+    P.bld_h2lo = std::isfinite(band) ? std::nextafterf((float)(h * h - band), 0.0f) : -1.0f;
+    P.bld_h2hi = std::isfinite(band) ? std::nextafterf((float)(h * h + band), INFINITY) : INFINITY;
   }
   P.h = (float)h;
   P.h2 = (float)(h * h);
