@@ -131,11 +131,8 @@ void launch_predict(const DevParams& P, PD* pd, const float4* vel, cudaStream_t 
 void launch_update_velocities(const DevParams& P, const PD* pd, float4* vel, cudaStream_t st,
                               const float* w_src = nullptr, uint4* nr = nullptr);
 void launch_update_positions(const DevParams& P, PD* pd, cudaStream_t st);
-// d.w and/or the record payload <- src[p] (a per-particle scalar for the
-// neighbour passes; null pd or nr skips it).
-void launch_pack_w(const DevParams& P, PD* pd, uint4* nr, const float* src, cudaStream_t st);
 // Neighbour records from particle records: canonical x* and payload
-// src[p * stride] (d.w when src is null).
+// src[p * stride] (0 when src is null).
 void launch_make_nr(const DevParams& P, const PD* pd, const float* src, uint4* nr,
                     cudaStream_t st, int stride = 1);
 // CalculateParticleCollisions seam on device double arrays.

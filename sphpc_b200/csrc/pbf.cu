@@ -530,9 +530,11 @@ __global__ void __launch_bounds__(kBlock) k_apply_dp(const DevParams P, const Pa
   ys = clamp_axis(ys, P.bmin[1], P.bmax[1], P.bmax_eps[1]);
   zs = clamp_axis(zs, P.bmin[2], P.bmax[2], P.bmax_eps[2]);
   if (SDF) sdf_collide(P, xs, ys, zs);
-  a.pd_out[p].d = make_float4(__double2float_rn(__dsub_rn(xs, (double)xp.x)),
-                              __double2float_rn(__dsub_rn(ys, (double)xp.y)),
-                              __double2float_rn(__dsub_rn(zs, (double)xp.z)), dp.w);
+  const float4 d = make_float4(__double2float_rn(__dsub_rn(xs, (double)xp.x)),
+                               __double2float_rn(__dsub_rn(ys, (double)xp.y)),
+                               __double2float_rn(__dsub_rn(zs, (double)xp.z)), dp.w);
+  a.pd_out[p].d = d;
+  a.nr_out[p] = make_nr(P, xstar_d(xp.x, d.x), xstar_d(xp.y, d.y), xstar_d(xp.z, d.z), 0.0f);
 }
 
 __global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
@@ -817,17 +819,8 @@ __global__ void __launch_bounds__(kBlock)
                         __double2float_rn(__dsub_rn(xstar_d(x.z, d.z), (double)nz)), d.w);
 }
 
-__global__ void __launch_bounds__(kBlock)
-    k_pack_w(const DevParams P, PD* pd, uint4* nr, const float* __restrict__ src) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const float w = src[p];
-  if (pd) pd[p].d.w = w;
-  if (nr) nr[p].w = __float_as_uint(w);
-}
-
 // 16-byte records from the particle records: canonical x* = x + d and the
-// payload src[p * stride] (d.w without src).
+// payload src[p * stride] (0 without src).
 __global__ void __launch_bounds__(kBlock)
     k_make_nr(const DevParams P, const PD* __restrict__ pd, const float* __restrict__ src,
               int stride, uint4* __restrict__ nr) {
@@ -835,7 +828,7 @@ __global__ void __launch_bounds__(kBlock)
   if (p >= P.n) return;
   const float4 x = pd[p].x, d = pd[p].d;
   nr[p] = make_nr(P, xstar_d(x.x, d.x), xstar_d(x.y, d.y), xstar_d(x.z, d.z),
-                  src ? src[(size_t)p * stride] : d.w);
+                  src ? src[(size_t)p * stride] : 0.0f);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -935,9 +928,6 @@ void launch_update_velocities(const DevParams& P, const PD* pd, float4* vel, cud
 }
 void launch_update_positions(const DevParams& P, PD* pd, cudaStream_t st) {
   k_update_positions<<<grid_for(P.n), kBlock, 0, st>>>(P, pd);
-}
-void launch_pack_w(const DevParams& P, PD* pd, uint4* nr, const float* src, cudaStream_t st) {
-  k_pack_w<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, nr, src);
 }
 void launch_make_nr(const DevParams& P, const PD* pd, const float* src, uint4* nr,
                     cudaStream_t st, int stride) {
