@@ -35,6 +35,8 @@ UNIT = "particle-steps/s"
 # reference-layout stage: x* and cell in, one count byte and ~30 four-byte
 # list entries out.
 STAGE_BYTES = {
+    "count_cells": 76,                      # r record 32, v 16, id 4, key, rank 4 + 4; w key,
+                                            # rank, id, slot 16; + 12 per cell, added below
     "hash": 60,                             # r record {x, d} 32, v 16, id 4; w key, slot 4 + 4
     "radix_sort": None,                     # 16 B per digit pass + 4, set below
     "cell_starts": 4,                       # + 8 per cell, added below
@@ -348,6 +350,8 @@ def run_ours(args, world, rank, local, dist):
             per = 16 * sim_passes(sim) + 4
         if name == "cell_starts":
             per = 4 + 8 * sim_cells(sim) / n
+        if name == "count_cells":
+            per += 12 * sim_cells(sim) / n
         if per is not None and cnt:
             avg_s = tot / cnt / 1e3
             bytes_launch = per * n
@@ -361,12 +365,12 @@ def run_ours(args, world, rank, local, dist):
                     "issue_active_ncu": ncu_stage(name).get("issue_active_pct"),
                     "avg_launch_ms": tot / cnt}
 
-    # the HBM-bound stages (hash, sort, cell starts, reorder), each against
+    # the HBM-bound stages (cells by counting, or hash, sort and cell starts; reorder), each against
     # the measured copy bandwidth on its algorithmic bytes
     hbm_class = {}
     if prof:
         peak, kind = peaks()
-        for name in ("hash", "radix_sort", "cell_starts", "reorder"):
+        for name in ("count_cells", "hash", "radix_sort", "cell_starts", "reorder"):
             if name not in prof or not prof[name][0]:
                 continue
             cnt, tot = prof[name]
@@ -375,6 +379,8 @@ def run_ours(args, world, rank, local, dist):
                 per = 16 * sim_passes(sim) + 4
             if name == "cell_starts":
                 per = 4 + 8 * sim_cells(sim) / n
+            if name == "count_cells":
+                per += 12 * sim_cells(sim) / n
             gbs = per * n / (tot / cnt / 1e3) / 1e9
             hbm_class[name] = {"bytes_per_particle": per, "avg_launch_ms": tot / cnt,
                                "achieved_gbs": gbs, "frac": gbs / peak}

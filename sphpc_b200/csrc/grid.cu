@@ -80,6 +80,26 @@ __device__ __forceinline__ uint32_t pack_cell(const DevParams& P, int cx, int cy
   return (uint32_t)cx | ((uint32_t)cy << P.bx) | ((uint32_t)cz << (P.bx + P.by));
 }
 
+// Cell key of the particle in slot i (launch_hash).
+__device__ __forceinline__ uint32_t key_of(const DevParams& P, const PD* __restrict__ pd,
+                                           const float4* __restrict__ vel, int i, bool predict,
+                                           uint32_t* __restrict__ err) {
+  float4 x, dg;
+  ld_pd(pd, i, x, dg);
+  const float4 v = predict ? __ldg(vel + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 d;
+  double xs, ys, zs;
+  canonical_xstar(P, x, v, dg, predict, d, xs, ys, zs);
+  int cx, cy, cz;
+  grid_cell(P, xs, ys, zs, cx, cy, cz);
+  const uint32_t key = cell_key(P, cx, cy, cz);
+  if (key >= P.ncells || cx >= P.nx || cy >= P.ny || cz >= P.nz) {
+    atomicOr(err, kErrCellRange);
+    return P.ncells - 1;
+  }
+  return key;
+}
+
 __global__ void __launch_bounds__(kBlock)
     k_hash(const DevParams P, const PD* __restrict__ pd, const float4* __restrict__ vel,
            const uint32_t* __restrict__ ids,
@@ -90,19 +110,7 @@ __global__ void __launch_bounds__(kBlock)
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < P.n) {
-    float4 x, dg;
-    ld_pd(pd, i, x, dg);
-    const float4 v = predict ? __ldg(vel + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 d;
-    double xs, ys, zs;
-    canonical_xstar(P, x, v, dg, predict != 0, d, xs, ys, zs);
-    int cx, cy, cz;
-    grid_cell(P, xs, ys, zs, cx, cy, cz);
-    uint32_t key = cell_key(P, cx, cy, cz);
-    if (key >= P.ncells || cx >= P.nx || cy >= P.ny || cz >= P.nz) {
-      atomicOr(err, kErrCellRange);
-      key = P.ncells - 1;
-    }
+    const uint32_t key = key_of(P, pd, vel, i, predict != 0, err);
     const uint32_t id = __ldg(ids + i);
     keys_by_id[id] = key;
     loc_by_id[id] = (uint32_t)i;
@@ -113,16 +121,197 @@ __global__ void __launch_bounds__(kBlock)
     if (s_hist[k]) atomicAdd(hist + k, s_hist[k]);
 }
 
+// ---------------------------------------------------------------------------
+// Slots by counting: count the particles of every cell, scan the counts to the
+// cell starts, put every particle's id somewhere in its cell's range, and take
+// its slot from the ids of the range (a cell's particles stand in ascending id).
+//
+// The state lies in the slots of the step before, so everything here runs nearly
+// in order; the digit passes start from the order of the ids, which takes a
+// scattered write and a scattered read of every particle besides.
+// One step of 1,048,576 particles: hash, three digit passes, bounds and reorder
+// 143 us, these and the reorder 74 us; 4.2M: 353 and 221 us; 290k: 83 and 39;
+// 4096: 42 and 27.  Empty cells cost 12 bytes each here and 4 there: at 27 cells a
+// particle 182 us against 229 (1M particles), 64 against 98 (262k).
+//
+// The rank by comparing takes time with the square of a cell's particles: 262,144
+// in eight cells are ranked in 12.7 ms, in digit passes in 65 us.  A cell of more
+// than kCrowded sets *crowded, host memory, and the set goes over to the digit
+// passes when the host sees it; the slots are the same either way.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kCrowded = 1024;
+
+// keys[i] of slot i, and its rank among its cell's particles in the order that
+// the atomics happen to take.  The lanes of a cell share one atomic: eight
+// particles a cell stand side by side.
 __global__ void __launch_bounds__(kBlock)
-    k_reorder(const DevParams P, const uint32_t* __restrict__ sorted_ids,
-              const uint32_t* __restrict__ loc_by_id, const PD* __restrict__ pd_in,
+    k_count(const DevParams P, const PD* __restrict__ pd, const float4* __restrict__ vel,
+            uint32_t* __restrict__ keys, uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
+            int predict, uint32_t* __restrict__ err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned on = __ballot_sync(0xffffffffu, i < P.n);
+  if (i >= P.n) return;
+  const uint32_t key = key_of(P, pd, vel, i, predict != 0, err);
+  const unsigned same = __match_any_sync(on, key);
+  const int lane = threadIdx.x & 31, first = __ffs((int)same) - 1;
+  uint32_t base = 0;
+  if (lane == first) base = atomicAdd(count + key, (uint32_t)__popc(same));
+  base = __shfl_sync(same, base, first);
+  keys[i] = key;
+  rank[i] = base + (uint32_t)__popc(same & ((1u << lane) - 1u));
+}
+
+// Exclusive scan of cells[0..m) in place: blocks of kScanItems cells in the
+// order of a ticket, each adding what the blocks before it hold (state: one word
+// a block, its own sum or the sum up to it).  state[0] is the ticket.
+constexpr int kScanThreads = 256;
+constexpr int kScanPer = 16;
+constexpr int kScanItems = kScanThreads * kScanPer;
+constexpr unsigned long long kScanSum = 1ull << 62, kScanPrefix = 2ull << 62;
+
+__device__ __forceinline__ unsigned long long ld_state(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_state(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_counts(uint32_t* __restrict__ cells, uint32_t m, unsigned long long* __restrict__ state,
+                  volatile uint32_t* crowded, uint32_t* __restrict__ err) {
+  __shared__ uint32_t s_warp[kScanThreads / 32];
+  __shared__ uint32_t s_block, s_before;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_block = (uint32_t)atomicAdd(state, 1ull);
+  __syncthreads();
+  const uint32_t block = s_block;
+  unsigned long long* mine = state + 1 + block;
+  const uint64_t c0 = (uint64_t)block * kScanItems + (uint64_t)threadIdx.x * kScanPer;
+  uint32_t v[kScanPer];
+  if (c0 + kScanPer <= m) {
+#pragma unroll
+    for (int u = 0; u < kScanPer; u += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(cells + c0 + u);
+      v[u] = q.x;
+      v[u + 1] = q.y;
+      v[u + 2] = q.z;
+      v[u + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < kScanPer; ++u) v[u] = c0 + u < m ? cells[c0 + u] : 0u;
+  }
+  uint32_t sum = 0, most = 0;
+#pragma unroll
+  for (int u = 0; u < kScanPer; ++u) {
+    const uint32_t x = v[u];
+    most = max(most, x);
+    v[u] = sum;
+    sum += x;
+  }
+  if (most > kCrowded) *crowded = 1u;
+  uint32_t upto = sum;
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, upto, k);
+    if (lane >= k) upto += y;
+  }
+  if (lane == 31) s_warp[warp] = upto;
+  __syncthreads();
+  uint32_t before = upto - sum, total = 0;
+#pragma unroll
+  for (int w = 0; w < kScanThreads / 32; ++w) {
+    if (w < warp) before += s_warp[w];
+    total += s_warp[w];
+  }
+  if (warp == 0) {
+    uint32_t ahead = 0;
+    if (block > 0) {
+      if (lane == 0) st_state(mine, kScanSum | total);
+      // 32 blocks back at a time until one that knows its prefix
+      for (int64_t b = (int64_t)block - 1 - lane, spins = 0;;) {
+        const unsigned long long q = b >= 0 ? ld_state(state + 1 + b) : kScanPrefix;
+        const unsigned unknown = __ballot_sync(0xffffffffu, q < kScanSum);
+        const unsigned prefix = __ballot_sync(0xffffffffu, q >= kScanPrefix);
+        // lanes up to the nearest prefix count; all of them must be known
+        const int last = prefix ? __ffs((int)prefix) - 1 : 31;
+        if (unknown & (0xffffffffu >> (31 - last))) {
+          if (++spins > (1 << 22)) {
+            if (lane == 0) atomicOr(err, kErrScanSpin);
+            break;
+          }
+          continue;
+        }
+        uint32_t x = lane <= last ? (uint32_t)q : 0u;
+#pragma unroll
+        for (int k = 16; k; k >>= 1) x += __shfl_xor_sync(0xffffffffu, x, k);
+        ahead += x;
+        if (prefix) break;
+        b -= 32;
+      }
+    }
+    if (lane == 0) {
+      st_state(mine, kScanPrefix | (uint32_t)(ahead + total));
+      s_before = ahead;
+    }
+  }
+  __syncthreads();
+  before += s_before;
+  if (c0 + kScanPer <= m) {
+#pragma unroll
+    for (int u = 0; u < kScanPer; u += 4)
+      *reinterpret_cast<uint4*>(cells + c0 + u) =
+          make_uint4(before + v[u], before + v[u + 1], before + v[u + 2], before + v[u + 3]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < kScanPer; ++u)
+      if (c0 + u < m) cells[c0 + u] = before + v[u];
+  }
+}
+
+// Id and old slot of every particle into its cell's range.
+__global__ void __launch_bounds__(kBlock)
+    k_place(int n, const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ keys,
+            const uint32_t* __restrict__ rank, const uint32_t* __restrict__ ids,
+            uint32_t* __restrict__ cell_ids, uint32_t* __restrict__ cell_src) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t j = min(__ldg(cstart + __ldg(keys + i)) + __ldg(rank + i), (uint32_t)n - 1u);
+  cell_ids[j] = __ldg(ids + i);
+  cell_src[j] = (uint32_t)i;
+}
+
+// Keys of the slots from the cell starts.
+__global__ void __launch_bounds__(kBlock)
+    k_slot_keys(const uint32_t* __restrict__ cstart, uint32_t ncells, uint32_t* __restrict__ keys) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncells) return;
+  for (uint32_t j = cstart[c]; j < cstart[c + 1]; ++j) keys[j] = c;
+}
+
+template <bool COUNTED>
+__global__ void __launch_bounds__(kBlock)
+    k_reorder(const DevParams P, const SlotOrder o, const PD* __restrict__ pd_in,
               const float4* __restrict__ vel_in, PD* __restrict__ pd_out,
               float4* __restrict__ vel_out, float4* __restrict__ xsa, uint4* __restrict__ nr_out,
               uint32_t* __restrict__ cellp, int predict, int move_vel, ReorderExtra ex) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= P.n) return;
-  const uint32_t id = __ldg(sorted_ids + j);
-  const uint32_t src = __ldg(loc_by_id + id);
+  const uint32_t id = __ldg(o.ids + j);
+  uint32_t src;
+  if (COUNTED) {
+    src = __ldg(o.src + j);
+    const uint32_t key = __ldg(o.keys + src);
+    const uint32_t b = __ldg(o.cstart + key), e = __ldg(o.cstart + key + 1);
+    uint32_t at = b;
+    for (uint32_t k = b; k < e; ++k) at += __ldg(o.ids + k) < id ? 1u : 0u;
+    j = (int)min(at, (uint32_t)P.n - 1u);
+    o.ids_out[j] = id;
+  } else {
+    src = __ldg(o.src + id);
+  }
   float4 x, dg;
   ld_pd(pd_in, (int)src, x, dg);
   float4 v = (predict || move_vel) ? __ldg(vel_in + src) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -696,15 +885,49 @@ void launch_hash(const DevParams& P, const PD* pd, const float4* vel, const uint
                                            passes, predict ? 1 : 0, err);
 }
 
-void launch_reorder(const DevParams& P, const uint32_t* sorted_ids, const uint32_t* loc_by_id,
-                    const PD* pd_in, const float4* vel_in, PD* pd_out, float4* vel_out,
-                    float4* xsa, uint4* nr_out, uint32_t* cellp, bool predict, bool move_vel,
-                    const ReorderExtra* extra, cudaStream_t st) {
+size_t cell_table_words(uint32_t ncells) {
+  // cstart[0..C], then the scan's ticket and block states
+  return (((size_t)ncells + 2) & ~(size_t)1) + 2 * (2 + (size_t)ncells / kScanItems + 1);
+}
+
+bool counts_cells(int n, uint32_t ncells) {
+  return n > 0 && (uint64_t)ncells <= 32ull * (uint64_t)n;
+}
+
+int launch_count_cells(const DevParams& P, const PD* pd, const float4* vel, const uint32_t* ids,
+                       uint32_t* cstart, uint32_t* keys, uint32_t* rank, uint32_t* cell_ids,
+                       uint32_t* cell_src, bool predict, uint32_t* crowded, uint32_t* err,
+                       cudaStream_t st) {
+  const uint32_t m = P.ncells + 1;
+  unsigned long long* state =
+      reinterpret_cast<unsigned long long*>(cstart + (((size_t)P.ncells + 2) & ~(size_t)1));
+  cudaMemsetAsync(cstart, 0, cell_table_words(P.ncells) * sizeof(uint32_t), st);
+  k_count<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, vel, keys, rank, cstart, predict ? 1 : 0, err);
+  k_scan_counts<<<(int)(((uint64_t)m + kScanItems - 1) / kScanItems), kScanThreads, 0, st>>>(
+      cstart, m, state, crowded, err);
+  k_place<<<grid_for(P.n), kBlock, 0, st>>>(P.n, cstart, keys, rank, ids, cell_ids, cell_src);
+  return 3;
+}
+
+void launch_slot_keys(const uint32_t* cstart, uint32_t ncells, uint32_t* keys, cudaStream_t st) {
+  k_slot_keys<<<(int)(((uint64_t)ncells + kBlock - 1) / kBlock), kBlock, 0, st>>>(cstart, ncells,
+                                                                                 keys);
+}
+
+void launch_reorder(const DevParams& P, const SlotOrder& order, const PD* pd_in,
+                    const float4* vel_in, PD* pd_out, float4* vel_out, float4* xsa, uint4* nr_out,
+                    uint32_t* cellp, bool predict, bool move_vel, const ReorderExtra* extra,
+                    cudaStream_t st) {
   ReorderExtra ex = {};
   if (extra) ex = *extra;
-  k_reorder<<<grid_for(P.n), kBlock, 0, st>>>(P, sorted_ids, loc_by_id, pd_in, vel_in, pd_out,
-                                              vel_out, xsa, nr_out, cellp, predict ? 1 : 0,
-                                              move_vel ? 1 : 0, ex);
+  if (order.keys)
+    k_reorder<true><<<grid_for(P.n), kBlock, 0, st>>>(P, order, pd_in, vel_in, pd_out, vel_out, xsa,
+                                                      nr_out, cellp, predict ? 1 : 0,
+                                                      move_vel ? 1 : 0, ex);
+  else
+    k_reorder<false><<<grid_for(P.n), kBlock, 0, st>>>(P, order, pd_in, vel_in, pd_out, vel_out,
+                                                       xsa, nr_out, cellp, predict ? 1 : 0,
+                                                       move_vel ? 1 : 0, ex);
 }
 
 // Up to kBoundsMaxCells cells the bounds kernel writes the table in one launch

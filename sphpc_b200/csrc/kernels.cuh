@@ -25,7 +25,34 @@ void launch_hash(const DevParams& P, const PD* pd, const float4* vel, const uint
                  uint32_t* keys_by_id, uint32_t* loc_by_id, uint32_t* hist, int passes,
                  bool predict, uint32_t* err, cudaStream_t st);
 
-// Reorder gather: new slot j takes particle sorted_ids[j] from its old slot.
+// The same by counting, for grids of up to 32 cells a particle
+// (counts_cells): the keys in slot order, the cell start table, and every
+// particle's id and old slot somewhere in its cell's range (cell_ids, cell_src).
+// cstart has cell_table_words(C) words; rank is scratch; *crowded (host memory)
+// becomes 1 when a cell holds so many that digit passes are faster.  Returns the kernels
+// launched.
+size_t cell_table_words(uint32_t ncells);
+bool counts_cells(int n, uint32_t ncells);
+int launch_count_cells(const DevParams& P, const PD* pd, const float4* vel, const uint32_t* ids,
+                       uint32_t* cstart, uint32_t* keys, uint32_t* rank, uint32_t* cell_ids,
+                       uint32_t* cell_src, bool predict, uint32_t* crowded, uint32_t* err,
+                       cudaStream_t st);
+// keys[j] of every slot from the cell start table.
+void launch_slot_keys(const uint32_t* cstart, uint32_t ncells, uint32_t* keys, cudaStream_t st);
+
+// Where the reorder finds its particles.  Without keys: slot j takes particle
+// ids[j] from old slot src[id].  With keys (those of the old slots): ids and src
+// stand in the ranges of their cells in any order, and the new slots' ids go to
+// ids_out.
+struct SlotOrder {
+  const uint32_t* ids;
+  const uint32_t* src;
+  const uint32_t* keys;
+  const uint32_t* cstart;
+  uint32_t* ids_out;
+};
+
+// Reorder gather: every particle from its old slot to its new one.
 // predict: recompute x* from x and v (+gravity) as launch_hash did, else
 // gather d.  Writes the records, x* as FP32 (xsa) and cellp (packed cell of
 // x*).  Optional extra float4 / float fields are gathered too (nullptr to
@@ -39,10 +66,10 @@ struct ReorderExtra {
   const float* carry_src;
   uint4* nr_carry;
 };
-void launch_reorder(const DevParams& P, const uint32_t* sorted_ids, const uint32_t* loc_by_id,
-                    const PD* pd_in, const float4* vel_in, PD* pd_out, float4* vel_out,
-                    float4* xsa, uint4* nr_out, uint32_t* cellp, bool predict, bool move_vel,
-                    const ReorderExtra* extra, cudaStream_t st);
+void launch_reorder(const DevParams& P, const SlotOrder& order, const PD* pd_in,
+                    const float4* vel_in, PD* pd_out, float4* vel_out, float4* xsa, uint4* nr_out,
+                    uint32_t* cellp, bool predict, bool move_vel, const ReorderExtra* extra,
+                    cudaStream_t st);
 
 // Cell start table cstart[0..C] from sorted keys (lower bounds; cstart[C]=n).
 // gaps: worklist scratch of >= n + 2 + C/4096 + 2 uint4 entries; gap_count:

@@ -95,7 +95,7 @@ class DeviceSim {
   float4 *color_alt = nullptr, *omega_alt = nullptr, *dp_alt = nullptr;
   float *rho_alt = nullptr, *lam_alt = nullptr;
   uint32_t *ids = nullptr, *ids_spare = nullptr, *keys_by_id = nullptr, *loc_by_id = nullptr;
-  uint32_t* keys_sorted = nullptr;  // view into keys_by_id or sort.keys_alt
+  uint32_t* keys_sorted = nullptr;  // view into keys_by_id or sort.keys_alt; null: not made
   uint32_t *cellp = nullptr, *nbr = nullptr, *cstart = nullptr;
   float4* xsa = nullptr;
   TileInfo* tiles = nullptr;  // of the current lists
@@ -110,6 +110,7 @@ class DeviceSim {
   // transfers run at full link speed); released in release()
   std::vector<void*> pinned;
   bool nbr_valid = false;
+  uint32_t* crowded = nullptr;   // page-locked: set by the device (launch_count_cells)
 
   MlpState mlp{};
   uint4 *nr = nullptr, *nr_alt = nullptr;  // 16-byte neighbour records (x* fixed point, payload)
@@ -210,6 +211,8 @@ class DeviceSim {
     ev_pool.clear();
     dfree(arena);
     arena_bytes = 0;
+    if (crowded) cudaFreeHost(crowded);
+    crowded = nullptr;
   }
 
   // Every array of a particle set, to `take(pointer, count)` in a fixed order.
@@ -260,6 +263,8 @@ class DeviceSim {
     }));
     const size_t aux = sort_aux_words(cap);
     sort_layout(sort, sort_aux);
+    SPHPC_CK(cudaHostAlloc(&crowded, sizeof(uint32_t), cudaHostAllocDefault));
+    *crowded = 0;
     SPHPC_CK(cudaMemsetAsync(ncount, 0, c, stream));
     SPHPC_CK(cudaMemsetAsync(small, 0, 8 * sizeof(uint32_t), stream));
     SPHPC_CK(cudaMemsetAsync(sort_aux, 0, aux * sizeof(uint32_t), stream));
@@ -329,7 +334,7 @@ class DeviceSim {
     nx = nnx; ny = nny; nz = nnz; C = CC; bx = bxx; by = byy;
     passes = (bits_for(C - 1) + kRadixBits - 1) / kRadixBits;
     if (passes > kMaxPasses) passes = kMaxPasses;
-    SPHPC_RC(dalloc(&cstart, (size_t)C + 1));
+    SPHPC_RC(dalloc(&cstart, cell_table_words(C)));
     dfree(gaps);
     SPHPC_RC(dalloc(&gaps, (size_t)cap + 4 + C / 4096));
     SPHPC_CK(cudaMemsetAsync(cstart, 0, sizeof(uint32_t) * ((size_t)C + 1), stream));
@@ -585,32 +590,44 @@ int DeviceSim::slab_setup(uint32_t first_gid, double lo, double hi, bool has_lef
 int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool move_vel,
                               const float* carry_src, uint4* carry_out) {
   if (!grid_ready) return set_error(SPHPC_ENOTREADY, "neighbour grid not initialised");
-  {
-    Scope sc(this, "hash");
-    SPHPC_CK(sort_clear(sort, n, passes, stream));
-    launch_hash(P, pd, vel, ids, keys_by_id, loc_by_id, sort.hist, passes, predict, err(),
-                stream);
-    launches += 1;
-  }
-  uint32_t *K = nullptr, *R = nullptr;
-  {
-    Scope sc(this, "radix_sort");
-    const cudaError_t e = radix_sort_pairs(keys_by_id, ids_spare, n, passes, sort, stream, true,
-                                           true, false, &K, &R);
-    if (e != cudaSuccess)
-      return set_error(SPHPC_ECUDA, "radix sort: %s", cudaGetErrorString(e));
-    launches += (unsigned)passes;
-  }
-  keys_sorted = K;
-  {
-    Scope sc(this, "cell_starts");
-    launches += launch_cell_starts(K, n, C, cstart, gaps, gap_count(), err(), stream);
+  if (full) SPHPC_RC(ensure_full_alts());
+  SlotOrder order{};
+  uint32_t* R = nullptr;
+  if (counts_cells(n, C) && !*static_cast<volatile uint32_t*>(crowded)) {
+    Scope sc(this, "count_cells");
+    launches += launch_count_cells(P, pd, vel, ids, cstart, keys_by_id, loc_by_id, sort.keys_alt,
+                                   sort.vals_alt, predict, crowded, err(), stream);
+    R = ids_spare;
+    order = SlotOrder{sort.keys_alt, sort.vals_alt, keys_by_id, cstart, R};
+    keys_sorted = nullptr;
+  } else {
+    uint32_t* K = nullptr;
+    {
+      Scope sc(this, "hash");
+      SPHPC_CK(sort_clear(sort, n, passes, stream));
+      launch_hash(P, pd, vel, ids, keys_by_id, loc_by_id, sort.hist, passes, predict, err(),
+                  stream);
+      launches += 1;
+    }
+    {
+      Scope sc(this, "radix_sort");
+      const cudaError_t e = radix_sort_pairs(keys_by_id, ids_spare, n, passes, sort, stream, true,
+                                             true, false, &K, &R);
+      if (e != cudaSuccess)
+        return set_error(SPHPC_ECUDA, "radix sort: %s", cudaGetErrorString(e));
+      launches += (unsigned)passes;
+    }
+    keys_sorted = K;
+    {
+      Scope sc(this, "cell_starts");
+      launches += launch_cell_starts(K, n, C, cstart, gaps, gap_count(), err(), stream);
+    }
+    order = SlotOrder{R, loc_by_id, nullptr, nullptr, nullptr};
   }
   {
     Scope sc(this, "reorder");
     ReorderExtra ex{};
     if (full) {
-      SPHPC_RC(ensure_full_alts());
       ex.in4[0] = color; ex.out4[0] = color_alt;
       ex.in4[1] = omega; ex.out4[1] = omega_alt;
       ex.in4[2] = dp; ex.out4[2] = dp_alt;
@@ -620,7 +637,7 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
     ex.carry_src = carry_src;
     ex.nr_carry = carry_src ? carry_out : nullptr;
     const bool mv = move_vel || full;
-    launch_reorder(P, R, loc_by_id, pd, vel, pd_alt, vel_alt, xsa, nr, cellp, predict, mv, &ex,
+    launch_reorder(P, order, pd, vel, pd_alt, vel_alt, xsa, nr, cellp, predict, mv, &ex,
                    stream);
     launches += 1;
     std::swap(pd, pd_alt);
@@ -1459,7 +1476,11 @@ int sphpc_get_neighbor_buckets(const struct Particles* particles, unsigned int* 
 int sphpc_get_cell_data(const struct Particles* particles, unsigned int* hash_values,
                         unsigned int* particle_ids, unsigned int* start_indices) {
   SPHPC_SIM(s, particles);
-  if (!s->nbr_valid || !s->keys_sorted) return set_error(SPHPC_ENOTREADY, "no cell data yet");
+  if (!s->nbr_valid) return set_error(SPHPC_ENOTREADY, "no cell data yet");
+  if (hash_values && !s->keys_sorted) {
+    s->keys_sorted = s->sort.keys_alt;
+    launch_slot_keys(s->cstart, s->C, s->keys_sorted, s->stream);
+  }
   if (hash_values)
     SPHPC_CK(cudaMemcpyAsync(hash_values, s->keys_sorted, sizeof(uint32_t) * s->n,
                              cudaMemcpyDeviceToHost, s->stream));

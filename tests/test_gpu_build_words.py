@@ -51,6 +51,29 @@ def test_buckets_of_dense_rows(tmp_path, dims, scale):
         assert sim.device_errors() == 0
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [0.05, 0.2])
+def test_crowded_cells_keep_their_order(tmp_path, scale):
+    """4913 particles in one cell (and in eight): the slots by counting and, once
+    the host has seen the crowded cell, by digit passes are the oracle's."""
+    with scene(tmp_path, (17, 17, 17)) as sim:
+        rng = np.random.default_rng(3)
+        pos = {f: (scale * rng.permutation(sim.host(f)) + 0.1).astype(np.float32).astype(np.float64)
+               for f in ("x", "y", "z")}
+        pos.update({f + "_star": v for f, v in pos.items()})
+        sim.push(pos)
+        o = oracle_for(sim, sim.fetch())
+        o.call("find_all_neighbors")
+        ocnt, onbr = o.neighbor_lists()
+        for _ in range(3):
+            sim.find_all_neighbors()
+            cnt, nbr = sim.neighbor_buckets()
+            np.testing.assert_array_equal(cnt, ocnt)
+            used = np.arange(nbr.shape[1])[None, :] < cnt[:, None]
+            np.testing.assert_array_equal(np.where(used, nbr, 0), np.where(used, onbr, 0))
+        assert sim.device_errors() == 0
+
+
 @pytest.mark.parametrize("h", [2.0, 1.0, 0.0125, 3.0])
 @pytest.mark.parametrize("cells", [1, 37, 128, 384, 768, 2000])
 def test_band_covers_the_rounding_of_its_grid(h, cells):
