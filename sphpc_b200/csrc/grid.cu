@@ -810,6 +810,7 @@ __global__ void __launch_bounds__(kTileSlots, 7)
                 axis_regular(xstar_d(xp.z, dp.z), P.hd, cz, P.nz);
     }
   }
+  if (p == 0) V.err[kGridBarrier] = 0;  // (for the solve of this step)
   if (threadIdx.x < 32) tile_ranges(P, V, cellp, first, min(first + kTileSlots, P.n) - 1, s_info);
   const bool all_regular = __syncthreads_and(regular ? 1 : 0) != 0;
   const int total = s_info.total;

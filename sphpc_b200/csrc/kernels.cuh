@@ -114,6 +114,27 @@ struct PassArgs {
   int acc_add;         // 1: add to lam_acc, 0: start it with this pass
 };
 
+// The solve of a set in one cooperative launch: `iterations` density and
+// position passes from the records nr and the particle records pd, with the
+// velocities of the last; writes nr (payload: the density), rho, pd_out and
+// vel_out.  nr_lam is scratch.  Sets of up to four blocks an SM (75,776 particles
+// on 148 SMs): with more registers a thread than the single passes have.
+constexpr int kSolveIterations = 16;
+constexpr int kSolveBlocksPerSm = 4;
+struct SolveArgs {
+  const PD* pd;
+  PD* pd_out;
+  uint4* nr;
+  uint4* nr_lam;
+  float* rho;
+  float4* vel_out;
+  int iterations;
+  float stiffness[kSolveIterations];
+};
+// The largest set that it takes on this device (0: none).
+int solve_max_particles(const DevParams& P, int device);
+cudaError_t launch_solve(const DevParams& P, const NbrView& V, const SolveArgs& a, cudaStream_t st);
+
 // Density (+lambda) pass: ComputeDensities (particles.c:461-514) and
 // ComputeLambda (:588-666).  mode 0: both (records with lambda in d.w to
 // pd_out, lam[] if set), mode 1: density only, mode 2: lambda only (reads

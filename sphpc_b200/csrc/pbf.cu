@@ -23,6 +23,8 @@
 // 2585 -> 2442.
 #include "kernels.cuh"
 
+#include <algorithm>
+
 namespace sphpc {
 
 namespace {
@@ -185,6 +187,79 @@ __device__ __forceinline__ void block_resid(double e, double* resid) {
   }
 }
 
+// Density (MODE 0, 1) and multiplier (MODE 0, 2, from rho) of particle p with
+// record rp over its list.
+template <int MODE, bool LIVE>
+__device__ __forceinline__ void density_lambda_of(const DevParams& P, const NbrView& V, bool tiled,
+                                                  const unsigned char* tile, const uint4* nr, int p,
+                                                  const uint4 rp, int cnt, const uint4 blk,
+                                                  float& rho, float& lam) {
+  // The loop keeps only what varies per pair: the density sums t^3 with
+  // t = h^2 - r^2 and the gradient sums c d with c = (h - r)^2 / r and d
+  // the pair difference, both in fixed-point units; the kernel norms, the
+  // mass and 2^-2k multiply the sums once afterwards.  The density sum is
+  // Kahan-compensated per batch: a batch's four terms are added pairwise
+  // (relative error at most 2 ulp of the batch sum, all terms >= 0) and the
+  // batch sum enters the compensated running sum.  Padding slots past the
+  // count are the pair (p, p): their density term is masked, their gradient
+  // terms carry d = 0.
+  float st = 0.0f, comp = 0.0f;
+  float sgx = 0.f, sgy = 0.f, sgz = 0.f, sC = 0.f;
+  visit<1, LIVE>(V, tiled, tile, nr, nullptr, p, cnt, blk,
+                  [&](const Batch<1>& q, int nvalid) {
+    float t[4], t2[4];
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {
+      const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
+      const uint64_t r2f = norm2_2(d);
+      if (MODE != 2) {
+        uint64_t tt = max2(f2_fma(f2_dup(-P.fx_inv2), r2f, f2_dup(P.h2)), 0.0f);
+        tt = f2_pack(u < nvalid ? f2_lo(tt) : 0.0f, u + 1 < nvalid ? f2_hi(tt) : 0.0f);
+        t[u] = f2_lo(tt);
+        t[u + 1] = f2_hi(tt);
+        tt = f2_mul(tt, tt);
+        t2[u] = f2_lo(tt);
+        t2[u + 1] = f2_hi(tt);
+      }
+      if (MODE != 1) {
+        // in fixed-point units: c_f = (h_f - r_f)^2 / r_f = 2^k c
+        const uint64_t r2c = max2(r2f, P.rmin2_fx);
+        const uint64_t rinv = rsqrt2(r2c);
+        const uint64_t hm = h_minus_r(P, r2c, rinv);
+        const uint64_t c = f2_mul(f2_mul(hm, hm), rinv);
+        const uint64_t cc = f2_mul(c, c);
+        // |c d|^2 = c^2 |d|^2: three fused accumulations and one for the norm
+        sgx = fmaf(f2_lo(c), f2_lo(d.x), sgx);
+        sgy = fmaf(f2_lo(c), f2_lo(d.y), sgy);
+        sgz = fmaf(f2_lo(c), f2_lo(d.z), sgz);
+        sC = fmaf(f2_lo(cc), f2_lo(r2f), sC);
+        sgx = fmaf(f2_hi(c), f2_hi(d.x), sgx);
+        sgy = fmaf(f2_hi(c), f2_hi(d.y), sgy);
+        sgz = fmaf(f2_hi(c), f2_hi(d.z), sgz);
+        sC = fmaf(f2_hi(cc), f2_hi(r2f), sC);
+      }
+    }
+    if (MODE != 2) {
+      // t0^3 + t1^3 + t2^3 + t3^3 as a chain of fused multiply-adds
+      const float yb = fmaf(t2[0], t[0], fmaf(t2[1], t[1],
+                            fmaf(t2[2], t[2], __fmul_rn(t2[3], t[3]))));
+      const float y = yb - comp;
+      const float s = st + y;
+      comp = (s - st) - y;
+      st = s;
+    }
+  });
+  if (MODE != 2) rho = fmaf(P.Wn_m, st - comp, P.W0m);
+  if (MODE != 1) {
+    // ComputeLambda's constraint (particles.c:616-617) in FP64
+    const float C = (float)fmax(__ddiv_rn((double)rho, P.rho0_d) - 1.0, 0.0);
+    const float g = P.DWn_m * P.fx_inv2;  // gradient scale (2^-2k is exact)
+    sC = __fadd_rn(sC, norm2(sgx, sgy, sgz));
+    sC *= (g * g) * P.inv_rho0_sq;
+    lam = -C / (sC + P.lambda_eps);
+  }
+}
+
 template <int MODE, bool RESID>
 __global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
     k_density_lambda(const DevParams P, const NbrView V, const PassArgs a) {
@@ -193,74 +268,11 @@ __global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
   const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
   SPHPC_PASS_READY();
   if (own) {
-    // The loop keeps only what varies per pair: the density sums t^3 with
-    // t = h^2 - r^2 and the gradient sums c d with c = (h - r)^2 / r and d
-    // the pair difference, both in fixed-point units; the kernel norms, the
-    // mass and 2^-2k multiply the sums once afterwards.  The density sum is
-    // Kahan-compensated per batch: a batch's four terms are added pairwise
-    // (relative error at most 2 ulp of the batch sum, all terms >= 0) and the
-    // batch sum enters the compensated running sum.  Padding slots past the
-    // count are the pair (p, p): their density term is masked, their gradient
-    // terms carry d = 0.
-    float st = 0.0f, comp = 0.0f;
-    float sgx = 0.f, sgy = 0.f, sgz = 0.f, sC = 0.f;
-    visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk,
-                    [&](const Batch<1>& q, int nvalid) {
-      float t[4], t2[4];
-#pragma unroll
-      for (int u = 0; u < 4; u += 2) {
-        const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
-        const uint64_t r2f = norm2_2(d);
-        if (MODE != 2) {
-          uint64_t tt = max2(f2_fma(f2_dup(-P.fx_inv2), r2f, f2_dup(P.h2)), 0.0f);
-          tt = f2_pack(u < nvalid ? f2_lo(tt) : 0.0f, u + 1 < nvalid ? f2_hi(tt) : 0.0f);
-          t[u] = f2_lo(tt);
-          t[u + 1] = f2_hi(tt);
-          tt = f2_mul(tt, tt);
-          t2[u] = f2_lo(tt);
-          t2[u + 1] = f2_hi(tt);
-        }
-        if (MODE != 1) {
-          // in fixed-point units: c_f = (h_f - r_f)^2 / r_f = 2^k c
-          const uint64_t r2c = max2(r2f, P.rmin2_fx);
-          const uint64_t rinv = rsqrt2(r2c);
-          const uint64_t hm = h_minus_r(P, r2c, rinv);
-          const uint64_t c = f2_mul(f2_mul(hm, hm), rinv);
-          const uint64_t cc = f2_mul(c, c);
-          // |c d|^2 = c^2 |d|^2: three fused accumulations and one for the norm
-          sgx = fmaf(f2_lo(c), f2_lo(d.x), sgx);
-          sgy = fmaf(f2_lo(c), f2_lo(d.y), sgy);
-          sgz = fmaf(f2_lo(c), f2_lo(d.z), sgz);
-          sC = fmaf(f2_lo(cc), f2_lo(r2f), sC);
-          sgx = fmaf(f2_hi(c), f2_hi(d.x), sgx);
-          sgy = fmaf(f2_hi(c), f2_hi(d.y), sgy);
-          sgz = fmaf(f2_hi(c), f2_hi(d.z), sgz);
-          sC = fmaf(f2_hi(cc), f2_hi(r2f), sC);
-        }
-      }
-      if (MODE != 2) {
-        // t0^3 + t1^3 + t2^3 + t3^3 as a chain of fused multiply-adds
-        const float yb = fmaf(t2[0], t[0], fmaf(t2[1], t[1],
-                              fmaf(t2[2], t[2], __fmul_rn(t2[3], t[3]))));
-        const float y = yb - comp;
-        const float s = st + y;
-        comp = (s - st) - y;
-        st = s;
-      }
-    });
-    float rho;
+    float rho = 0.0f, lam = 0.0f;
     if (MODE == 2) rho = a.rho[p];
-    if (MODE != 2) {
-      rho = fmaf(P.Wn_m, st - comp, P.W0m);
-      a.rho[p] = rho;
-    }
+    density_lambda_of<MODE, false>(P, V, tiled, tile, a.nr, p, rp, cnt, blk, rho, lam);
+    if (MODE != 2) a.rho[p] = rho;
     if (MODE != 1) {
-      // ComputeLambda's constraint (particles.c:616-617) in FP64
-      const float C = (float)fmax(__ddiv_rn((double)rho, P.rho0_d) - 1.0, 0.0);
-      const float g = P.DWn_m * P.fx_inv2;  // gradient scale (2^-2k is exact)
-      sC = __fadd_rn(sC, norm2(sgx, sgy, sgz));
-      sC *= (g * g) * P.inv_rho0_sq;
-      const float lam = -C / (sC + P.lambda_eps);
       if (a.nr_out) a.nr_out[p] = make_uint4(rp.x, rp.y, rp.z, __float_as_uint(lam));
       if (a.lam) a.lam[p] = lam;
     }
@@ -434,22 +446,20 @@ __global__ void k_accum_lambda(const uint4* __restrict__ rec, float s, float* __
   if (p < limit) target[p] = fmaf(s, __uint_as_float(rec[p].w), target[p]);
 }
 
-template <int MODE, int SCORR_N, bool SDF>
-__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
-    k_position(const DevParams P, const NbrView V, const PassArgs a) {
-  SPHPC_PASS_HEAD(1, a.nr, nullptr);
-  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
-  SPHPC_PASS_READY();
-  if (!own) return;
+// Displacement of particle p with record rp (payload lambda) over its list
+// (UpdateDPs), for the stiffness of the substep.
+template <int SCORR_N, bool LIVE>
+__device__ __forceinline__ float3 displacement_of(const DevParams& P, const NbrView& V, bool tiled,
+                                                  const unsigned char* tile, const uint4* nr, int p,
+                                                  const uint4 rp, int cnt, const uint4 blk,
+                                                  float stiffness) {
   const float lp = nr_w(rp);
-  float4 xp, dp;  // own particle record, loaded ahead of the neighbour loop
-  if (MODE == 0) ld_pd(a.pd, p, xp, dp);
   // sums of c d with c = (lambda_p + lambda_q + s_corr) (h - r)^2 / r and d
   // the pair difference, both in fixed-point units; the spiky norm, the mass
   // and 2^-2k multiply them once afterwards.  Every term carries d, so the batch's
   // padding slots (q = p, d = 0) add nothing and are not masked.
   float ax = 0.f, ay = 0.f, az = 0.f;
-  visit<1>(V, tiled, tile, a.nr, nullptr, p, cnt, blk, [&](const Batch<1>& q, int) {
+  visit<1, LIVE>(V, tiled, tile, nr, nullptr, p, cnt, blk, [&](const Batch<1>& q, int) {
 #pragma unroll
     for (int u = 0; u < 4; u += 2) {
       const Pair2 d = diff2(rp, q.r[u], q.r[u + 1]);
@@ -482,38 +492,187 @@ __global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
       az = fmaf(f2_hi(c), f2_hi(d.z), az);
     }
   });
-  const float s = a.stiffness * P.inv_rho0 * (P.DWn_m * P.fx_inv2);
-  const float dpx = ax * s, dpy = ay * s, dpz = az * s;
-  if (MODE == 1) {
-    a.dp[p] = make_float4(dpx, dpy, dpz, 0.0f);
-    return;
-  }
-  double xs = __dadd_rn(xstar_d(xp.x, dp.x), (double)dpx);
-  double ys = __dadd_rn(xstar_d(xp.y, dp.y), (double)dpy);
-  double zs = __dadd_rn(xstar_d(xp.z, dp.z), (double)dpz);
+  const float s = stiffness * P.inv_rho0 * (P.DWn_m * P.fx_inv2);
+  return make_float3(ax * s, ay * s, az * s);
+}
+
+// x* of the record {xp, d} moved by dp (UpdatePositionStars): the new d, with
+// rho as its payload, and the exact x* - x.
+template <bool SDF>
+__device__ __forceinline__ float4 move_star(const DevParams& P, const float4 xp, const float4 d,
+                                            const float3 dp, float rho, double& ex, double& ey,
+                                            double& ez) {
+  double xs = __dadd_rn(xstar_d(xp.x, d.x), (double)dp.x);
+  double ys = __dadd_rn(xstar_d(xp.y, d.y), (double)dp.y);
+  double zs = __dadd_rn(xstar_d(xp.z, d.z), (double)dp.z);
   xs = clamp_axis(xs, P.bmin[0], P.bmax[0], P.bmax_eps[0]);
   ys = clamp_axis(ys, P.bmin[1], P.bmax[1], P.bmax_eps[1]);
   zs = clamp_axis(zs, P.bmin[2], P.bmax[2], P.bmax_eps[2]);
   if (SDF) sdf_collide(P, xs, ys, zs);
-  const double ex = __dsub_rn(xs, (double)xp.x), ey = __dsub_rn(ys, (double)xp.y),
-               ez = __dsub_rn(zs, (double)xp.z);
-  const float rho_p = a.rho[p];
-  const float4 dn = make_float4(__double2float_rn(ex), __double2float_rn(ey),
-                                __double2float_rn(ez), rho_p);
-  st_pd(a.pd_out, p, xp, dn);
-  // the record carries the canonical x* = x + d of what was just stored
-  a.nr_out[p] = make_nr(P, xstar_d(xp.x, dn.x), xstar_d(xp.y, dn.y), xstar_d(xp.z, dn.z), rho_p);
-  if (a.lam_acc) a.lam_acc[p] = fmaf(a.stiffness, lp, a.acc_add ? a.lam_acc[p] : 0.0f);
-  if (a.last) {
-    // UpdateVelocities, particles.c:814-837
-    float vx = __double2float_rn(__ddiv_rn(ex, P.dt_d));
-    float vy = __double2float_rn(__ddiv_rn(ey, P.dt_d));
-    float vz = __double2float_rn(__ddiv_rn(ez, P.dt_d));
-    vx = fminf(fmaxf(vx, -P.v_max), P.v_max);
-    vy = fminf(fmaxf(vy, -P.v_max), P.v_max);
-    vz = fminf(fmaxf(vz, -P.v_max), P.v_max);
-    a.vel_out[p] = make_float4(vx, vy, vz, 0.0f);
+  ex = __dsub_rn(xs, (double)xp.x);
+  ey = __dsub_rn(ys, (double)xp.y);
+  ez = __dsub_rn(zs, (double)xp.z);
+  return make_float4(__double2float_rn(ex), __double2float_rn(ey), __double2float_rn(ez), rho);
+}
+
+// UpdateVelocities, particles.c:814-837
+__device__ __forceinline__ float4 velocity_of(const DevParams& P, double ex, double ey, double ez) {
+  float vx = __double2float_rn(__ddiv_rn(ex, P.dt_d));
+  float vy = __double2float_rn(__ddiv_rn(ey, P.dt_d));
+  float vz = __double2float_rn(__ddiv_rn(ez, P.dt_d));
+  vx = fminf(fmaxf(vx, -P.v_max), P.v_max);
+  vy = fminf(fmaxf(vy, -P.v_max), P.v_max);
+  vz = fminf(fmaxf(vz, -P.v_max), P.v_max);
+  return make_float4(vx, vy, vz, 0.0f);
+}
+
+// The record of the canonical x* = x + d.
+__device__ __forceinline__ uint4 record_of(const DevParams& P, const float4 xp, const float4 d) {
+  return make_nr(P, xstar_d(xp.x, d.x), xstar_d(xp.y, d.y), xstar_d(xp.z, d.z), d.w);
+}
+
+template <int MODE, int SCORR_N, bool SDF>
+__global__ void __launch_bounds__(kTileSlots, kMinBlocks1)
+    k_position(const DevParams P, const NbrView V, const PassArgs a) {
+  SPHPC_PASS_HEAD(1, a.nr, nullptr);
+  const uint4 rp = own ? ld_nr(a.nr, p) : make_uint4(0u, 0u, 0u, 0u);
+  SPHPC_PASS_READY();
+  if (!own) return;
+  float4 xp, d;  // own particle record, loaded ahead of the neighbour loop
+  if (MODE == 0) ld_pd(a.pd, p, xp, d);
+  const float3 dp = displacement_of<SCORR_N, false>(P, V, tiled, tile, a.nr, p, rp, cnt, blk,
+                                                    a.stiffness);
+  if (MODE == 1) {
+    a.dp[p] = make_float4(dp.x, dp.y, dp.z, 0.0f);
+    return;
   }
+  double ex, ey, ez;
+  const float4 dn = move_star<SDF>(P, xp, d, dp, a.rho[p], ex, ey, ez);
+  st_pd(a.pd_out, p, xp, dn);
+  // the record carries the canonical x* of what was just stored
+  a.nr_out[p] = record_of(P, xp, dn);
+  if (a.lam_acc) a.lam_acc[p] = fmaf(a.stiffness, nr_w(rp), a.acc_add ? a.lam_acc[p] : 0.0f);
+  if (a.last) a.vel_out[p] = velocity_of(P, ex, ey, ez);
+}
+
+// ---------------------------------------------------------------------------
+// The whole solve of a small set in one launch: every iteration's density and
+// position pass, with the blocks meeting between them.  A block keeps its slots:
+// records, multipliers, densities and positions of its particles stay in
+// registers, and a pass reads only its tile and its lists.
+//
+// Bound: latency.  A pass of a set that is resident at once is a chain of a
+// launch, the tile's ranges, the copies, the lists and the sums; the meeting takes
+// the place of the launch and the first loads.
+// Step of 4096 particles (200 steps after the dam broke, four iterations) 123 ->
+// 115 us, of 32,768 152 -> 138, of 68,921 178 -> 172; at the start of a scene 4096
+// 140 -> 121 us a step.  Larger sets fill the device with one pass and have their
+// own kernels (nine blocks an SM instead of four).
+// A cooperative launch, so every block is resident; the wait is bounded all
+// the same.  The records are written by other blocks while the kernel runs:
+// ordinary loads and fences on both sides of the meeting, also between the
+// ordinary stores and the bulk copies (fence.proxy.async).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool grid_meet(uint32_t* count, uint32_t target, bool wait) {
+  __shared__ int s_met;
+  asm volatile("fence.proxy.async;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    bool met = false;
+    for (int i = 0; wait && i < (1 << 20); ++i) {
+      uint32_t c;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+      if ((met = c >= target)) break;
+    }
+    __threadfence();
+    s_met = met ? 1 : 0;
+  }
+  __syncthreads();
+  asm volatile("fence.proxy.async;" ::: "memory");
+  return s_met != 0;
+}
+
+template <int SCORR_N, bool SDF>
+__global__ void __launch_bounds__(kTileSlots, 4)
+    k_solve(const DevParams P, const NbrView V, const SolveArgs a) {
+  extern __shared__ __align__(128) unsigned char tile[];
+  __shared__ __align__(8) uint64_t s_mbar;
+  __shared__ TileInfo s_info;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool own = p < P.n;
+  const int cnt = own ? (int)__ldg(V.ncount + p) : 0;
+  const uint4 blk = cnt > 0 ? nbr_block(V, p, 0) : make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x < sizeof(TileInfo) / sizeof(int))
+    reinterpret_cast<int*>(&s_info)[threadIdx.x] =
+        __ldg(reinterpret_cast<const int*>(V.tiles + blockIdx.x) + threadIdx.x);
+  if (threadIdx.x == 0) mbar_init1(&s_mbar);
+  uint4 rp = make_uint4(0u, 0u, 0u, 0u);
+  float4 xp = make_float4(0.f, 0.f, 0.f, 0.f), d = xp;
+  if (own) {
+    rp = a.nr[p];
+    ld_pd(a.pd, p, xp, d);
+  }
+  __syncthreads();
+  const bool tiled = s_info.total >= 0;
+  uint32_t* const count = V.err + kGridBarrier;
+  uint32_t target = 0, phase = 0;
+  bool good = true;  // the same in every thread of the block
+  // a pass's tile of `nr`; false: it did not arrive
+  auto fetch = [&](const uint4* nr) {
+    if (!tiled) return;
+    if (threadIdx.x == 0) mbar_expect(&s_mbar, (uint32_t)s_info.total * 16u);
+    __syncwarp();
+    if (threadIdx.x < 9) {
+      const int r = threadIdx.x, s = s_info.s[r], o = s_info.o[r],
+                e = r < 8 ? s_info.o[r + 1] : s_info.total;
+      if (e > o) bulk_load(tile + o * 16, nr + s, (uint32_t)(e - o) * 16u, &s_mbar);
+    }
+  };
+  auto arrived = [&]() {
+    if (!tiled) return true;
+    if (mbar_wait(&s_mbar, phase)) return true;
+    atomicOr(V.err, kErrTileWait);
+    mbar_wait(&s_mbar, phase);
+    return false;
+  };
+  auto meet = [&]() {
+    target += gridDim.x;
+    if (!grid_meet(count, target, good)) {
+      if (good && threadIdx.x == 0) atomicOr(V.err, kErrGridWait);
+      good = false;
+    }
+  };
+  double ex = 0.0, ey = 0.0, ez = 0.0;
+  float rho = 0.0f;
+  for (int it = 0; it < a.iterations; ++it) {
+    if (it > 0) meet();
+    fetch(a.nr);
+    bool here = arrived();
+    phase ^= 1u;
+    float lam = 0.0f;
+    if (own) {
+      density_lambda_of<0, true>(P, V, tiled, tile, a.nr, p, rp, here ? cnt : 0, blk, rho, lam);
+      rp.w = __float_as_uint(lam);
+      a.nr_lam[p] = rp;
+    }
+    meet();
+    fetch(a.nr_lam);
+    here = arrived();
+    phase ^= 1u;
+    if (own) {
+      const float3 dp = displacement_of<SCORR_N, true>(P, V, tiled, tile, a.nr_lam, p, rp,
+                                                       here ? cnt : 0, blk, a.stiffness[it]);
+      d = move_star<SDF>(P, xp, d, dp, rho, ex, ey, ez);
+      rp = record_of(P, xp, d);
+      a.nr[p] = rp;
+    }
+  }
+  if (!own) return;
+  a.rho[p] = rho;
+  st_pd(a.pd_out, p, xp, d);
+  a.vel_out[p] = velocity_of(P, ex, ey, ez);
 }
 
 template <bool SDF>
@@ -893,6 +1052,39 @@ void launch_position(const DevParams& P, const NbrView& V, const PassArgs& a, in
     else SPHPC_POS(1, -1, false);
   }
 #undef SPHPC_POS
+}
+
+namespace {
+using SolveKernel = void (*)(DevParams, NbrView, SolveArgs);
+SolveKernel solve_kernel(const DevParams& P) {
+  const int sn = P.scorr_k != 0.0f ? (P.scorr_n == 4 ? 4 : -1) : 0;
+  if (P.has_sdf) return sn == 0 ? k_solve<0, true> : sn == 4 ? k_solve<4, true> : k_solve<-1, true>;
+  return sn == 0 ? k_solve<0, false> : sn == 4 ? k_solve<4, false> : k_solve<-1, false>;
+}
+constexpr size_t kSolveTile = (size_t)kTileCap * 16;
+}  // namespace
+
+int solve_max_particles(const DevParams& P, int device) {
+  int sms = 0, blocks = 0, coop = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, solve_kernel(P), kTileSlots,
+                                                    kSolveTile) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return std::min(blocks, kSolveBlocksPerSm) * sms * kTileSlots;
+}
+
+cudaError_t launch_solve(const DevParams& P, const NbrView& V, const SolveArgs& a,
+                         cudaStream_t st) {
+  DevParams p = P;
+  NbrView v = V;
+  SolveArgs s = a;
+  void* args[] = {&p, &v, &s};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(solve_kernel(P)),
+                                     dim3(grid_for(P.n, kTileSlots)), dim3(kTileSlots), args,
+                                     kSolveTile, st);
 }
 
 void launch_apply_dp(const DevParams& P, const PassArgs& a, cudaStream_t st) {

@@ -110,6 +110,7 @@ class DeviceSim {
   // transfers run at full link speed); released in release()
   std::vector<void*> pinned;
   bool nbr_valid = false;
+  int solve_max[6] = {-1, -1, -1, -1, -1, -1};  // solve_max_particles by kernel; -1: not asked
   uint32_t* crowded = nullptr;   // page-locked: set by the device (launch_count_cells)
 
   MlpState mlp{};
@@ -824,6 +825,21 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
   // discarded) included, so that both arms of a comparison get the same work
   // budget.
   bool fused_velocity = false;
+  if (!adaptive && !collect && !carry_mode && !ready && iters == 0 && plain_cap > 0 &&
+      plain_cap <= kSolveIterations) {
+    const int variant = (P.has_sdf ? 3 : 0) + (P.scorr_k == 0.0f ? 0 : P.scorr_n == 4 ? 1 : 2);
+    if (solve_max[variant] < 0) solve_max[variant] = solve_max_particles(P, device);
+    if (n > 0 && n <= solve_max[variant]) {
+      Scope sc(this, "solve");
+      SolveArgs sa{pd, pd_alt, nr, nr_alt, rho, vel, plain_cap, {}};
+      for (int k = 0; k < plain_cap; ++k) sa.stiffness[k] = stiffness_of(solver.stiffness_k, k);
+      SPHPC_CK(launch_solve(P, V, sa, stream));
+      launches += 1;
+      std::swap(pd, pd_alt);
+      iters = plain = plain_cap;
+      fused_velocity = true;
+    }
+  }
   while (!converged && iters < plain_cap) {
     const uint4* src = ready;
     ready = nullptr;

@@ -121,7 +121,11 @@ enum : uint32_t {
   kErrScanSpin = 1u << 3,
   kErrNbrTail = 1u << 5,           // a list block's entries past the count are not p
   kErrTileWait = 1u << 6,          // the wait for a tile's bulk copies gave up
+  kErrGridWait = 1u << 7,          // the solve's wait for the other blocks gave up
 };
+
+// Word after the error bits that the blocks of the solve meet at.
+constexpr int kGridBarrier = 2;
 
 struct DevParams {
   int n;
@@ -242,22 +246,23 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Bounded wait for phase 0 of an mbarrier (~1e6 polls, each of which may
-// itself suspend the thread for a while).
-__device__ __forceinline__ bool mbar_wait0(uint64_t* mbar) {
+// Bounded wait for a phase (parity) of an mbarrier (~1e6 polls, each of which
+// may itself suspend the thread for a while).
+__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity) {
   const uint32_t addr = smem_addr(mbar);
   for (int i = 0; i < (1 << 20); ++i) {
     uint32_t ok;
     asm volatile(
-        "{\n.reg .pred P1;\nmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], 0;\n"
+        "{\n.reg .pred P1;\nmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n"
         "selp.b32 %0, 1, 0, P1;\n}\n"
         : "=r"(ok)
-        : "r"(addr)
+        : "r"(addr), "r"(parity)
         : "memory");
     if (ok) return true;
   }
   return false;
 }
+__device__ __forceinline__ bool mbar_wait0(uint64_t* mbar) { return mbar_wait(mbar, 0); }
 
 __device__ __forceinline__ void mbar_init1(uint64_t* mbar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mbar)));
@@ -337,9 +342,10 @@ struct Batch {
 // next list block is loaded before this one's bodies run.  (Eight entries a
 // round without the test between them measured 5% slower: more registers live
 // for no fewer wavefronts.)
-template <int NARR, class F>
+// LIVE: the records change while the kernel runs (ordinary loads, after a fence).
+template <int NARR, bool LIVE = false, class F>
 __device__ __forceinline__ void visit(const NbrView& v, bool tiled, const unsigned char* tile,
-                                      const uint4* __restrict__ nr, const float4* __restrict__ e,
+                                      const uint4* nr, const float4* __restrict__ e,
                                       int p, int cnt, uint4 blk, F&& f) {
   if (tiled) {
     auto load = [&](uint32_t w0, uint32_t w1) {
@@ -365,7 +371,7 @@ __device__ __forceinline__ void visit(const NbrView& v, bool tiled, const unsign
       Batch<NARR> b;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        b.r[u] = ld_nr(nr, q[u]);
+        b.r[u] = LIVE ? *(nr + q[u]) : ld_nr(nr, q[u]);
         if (NARR == 2) b.e[u] = __ldg(e + q[u]);
       }
       f(b, cnt - j0);
