@@ -782,10 +782,11 @@ __global__ void __launch_bounds__(kTileSlots, 7)
             uint32_t* __restrict__ nbr, uint8_t* __restrict__ ncount, TileInfo* __restrict__ tiles) {
   // the tile (its last group of four may read three records past it), or the
   // bases of the hit words of a block without one
-  __shared__ __align__(128) float4 s_tile[kTileCap + 4];
-  __shared__ uint32_t s_mask[(kWords + 1) * kTileSlots];
-  __shared__ uint16_t s_base[(kWords + 1) * kTileSlots];
-  static_assert(sizeof(int) * (kWords + 1) * kTileSlots <= sizeof(s_tile), "bases fit in the tile");
+  extern __shared__ __align__(128) float4 s_tile[];
+  uint32_t* const s_mask = reinterpret_cast<uint32_t*>(s_tile + V.cap + 4);
+  uint16_t* const s_base = reinterpret_cast<uint16_t*>(s_mask + (kWords + 1) * kTileSlots);
+  static_assert(sizeof(int) * (kWords + 1) * kTileSlots <= sizeof(float4) * kTileCap,
+                "bases fit in the tile");
   __shared__ TileInfo s_info;
   __shared__ int s_off[9];
   __shared__ __align__(8) uint64_t s_mbar;
@@ -814,7 +815,7 @@ __global__ void __launch_bounds__(kTileSlots, 7)
   if (threadIdx.x < 32) tile_ranges(P, V, cellp, first, min(first + kTileSlots, P.n) - 1, s_info);
   const bool all_regular = __syncthreads_and(regular ? 1 : 0) != 0;
   const int total = s_info.total;
-  const bool tiled = all_regular && total <= kTileCap;
+  const bool tiled = all_regular && total <= V.cap;
   if (threadIdx.x < 32) {
     const int r = threadIdx.x;
     if (r < 9) {
@@ -957,8 +958,11 @@ int launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint
 void launch_build_neighbors(const DevParams& P, const NbrView& V, const PD* pd,
                             const float4* xsa, const uint32_t* cellp, uint32_t* nbr,
                             uint8_t* ncount, TileInfo* tiles, cudaStream_t st) {
-  k_build<<<grid_for(P.n, kTileSlots), kTileSlots, 0, st>>>(P, V, pd, xsa, cellp, nbr, ncount,
-                                                            tiles);
+  const size_t bytes = (size_t)(V.cap + 4) * sizeof(float4) +
+                       (kWords + 1) * kTileSlots * (sizeof(uint32_t) + sizeof(uint16_t));
+  allow_shared(k_build, bytes);
+  k_build<<<grid_for(P.n, kTileSlots), kTileSlots, bytes, st>>>(P, V, pd, xsa, cellp, nbr, ncount,
+                                                                tiles);
 }
 
 void launch_export_buckets(const NbrView& V, const uint32_t* ids, uint32_t* nbr, int32_t* count,

@@ -131,8 +131,8 @@ struct SolveArgs {
   int iterations;
   float stiffness[kSolveIterations];
 };
-// The largest set that it takes on this device (0: none).
-int solve_max_particles(const DevParams& P, int device);
+// Whether it takes this set on this device.
+bool solve_fits(const DevParams& P, const NbrView& V, int device, int sms);
 cudaError_t launch_solve(const DevParams& P, const NbrView& V, const SolveArgs& a, cudaStream_t st);
 
 // Density (+lambda) pass: ComputeDensities (particles.c:461-514) and

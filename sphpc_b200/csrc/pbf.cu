@@ -300,7 +300,7 @@ template <bool RAW>
 __global__ void __launch_bounds__(kTileSlots, kMinBlocksFeatures)
     k_features(const DevParams P, const NbrView V, const PassArgs a, float* __restrict__ feat,
                __nv_bfloat16* __restrict__ xbf, const float* __restrict__ norm, int limit) {
-  __shared__ int s_slot[kTileCap];
+  __shared__ int s_slot[kTileCapMost];
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   const TileInfo* info = V.tiles + blockIdx.x;
   const int total = __ldg(&info->total);
@@ -1005,20 +1005,23 @@ __global__ void __launch_bounds__(kBlock)
 }  // namespace
 
 // Launch of a neighbour pass with the tiles of NARR arrays.
-#define SPHPC_COMMA ,
-#define SPHPC_PASS(NARR, kernel) \
-  kernel<<<grid_for(P.n, kTileSlots), kTileSlots, NARR * kTileCap * 16, st>>>(P, V, a)
+#define SPHPC_PASS(NARR, ...)                                                       \
+  do {                                                                              \
+    const size_t bytes = (size_t)NARR * V.cap * 16;                                 \
+    allow_shared(__VA_ARGS__, bytes);                                               \
+    __VA_ARGS__<<<grid_for(P.n, kTileSlots), kTileSlots, bytes, st>>>(P, V, a);     \
+  } while (0)
 
 void launch_density_lambda(const DevParams& P, const NbrView& V, const PassArgs& a, int mode,
                            bool residual, cudaStream_t st) {
   if (mode == 0) {
-    if (residual) SPHPC_PASS(1, k_density_lambda<0 SPHPC_COMMA true>);
-    else SPHPC_PASS(1, k_density_lambda<0 SPHPC_COMMA false>);
+    if (residual) SPHPC_PASS(1, k_density_lambda<0, true>);
+    else SPHPC_PASS(1, k_density_lambda<0, false>);
   } else if (mode == 1) {
-    if (residual) SPHPC_PASS(1, k_density_lambda<1 SPHPC_COMMA true>);
-    else SPHPC_PASS(1, k_density_lambda<1 SPHPC_COMMA false>);
+    if (residual) SPHPC_PASS(1, k_density_lambda<1, true>);
+    else SPHPC_PASS(1, k_density_lambda<1, false>);
   } else {
-    SPHPC_PASS(1, k_density_lambda<2 SPHPC_COMMA false>);
+    SPHPC_PASS(1, k_density_lambda<2, false>);
   }
 }
 
@@ -1041,7 +1044,7 @@ void launch_position(const DevParams& P, const NbrView& V, const PassArgs& a, in
   const int sn = P.scorr_k != 0.0f ? (P.scorr_n == 4 ? 4 : -1) : 0;
   const bool sdf = P.has_sdf != 0;
 #define SPHPC_POS(M, N, S) \
-  SPHPC_PASS(1, k_position<M SPHPC_COMMA N SPHPC_COMMA S>)
+  SPHPC_PASS(1, k_position<M, N, S>)
   if (mode == 0) {
     if (sn == 0) { if (sdf) SPHPC_POS(0, 0, true); else SPHPC_POS(0, 0, false); }
     else if (sn == 4) { if (sdf) SPHPC_POS(0, 4, true); else SPHPC_POS(0, 4, false); }
@@ -1061,19 +1064,20 @@ SolveKernel solve_kernel(const DevParams& P) {
   if (P.has_sdf) return sn == 0 ? k_solve<0, true> : sn == 4 ? k_solve<4, true> : k_solve<-1, true>;
   return sn == 0 ? k_solve<0, false> : sn == 4 ? k_solve<4, false> : k_solve<-1, false>;
 }
-constexpr size_t kSolveTile = (size_t)kTileCap * 16;
 }  // namespace
 
-int solve_max_particles(const DevParams& P, int device) {
-  int sms = 0, blocks = 0, coop = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, solve_kernel(P), kTileSlots,
-                                                    kSolveTile) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return std::min(blocks, kSolveBlocksPerSm) * sms * kTileSlots;
+bool solve_fits(const DevParams& P, const NbrView& V, int device, int sms) {
+  const int per_sm = (grid_for(P.n, kTileSlots) + sms - 1) / sms;
+  if (P.n <= 0 || per_sm > kSolveBlocksPerSm) return false;
+  const size_t bytes = (size_t)V.cap * 16;
+  int blocks = 0, coop = 0;
+  allow_shared(solve_kernel(P), bytes);
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, solve_kernel(P), kTileSlots, bytes) ==
+          cudaSuccess)
+    return per_sm <= blocks;
+  cudaGetLastError();
+  return false;
 }
 
 cudaError_t launch_solve(const DevParams& P, const NbrView& V, const SolveArgs& a,
@@ -1084,7 +1088,7 @@ cudaError_t launch_solve(const DevParams& P, const NbrView& V, const SolveArgs& 
   void* args[] = {&p, &v, &s};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(solve_kernel(P)),
                                      dim3(grid_for(P.n, kTileSlots)), dim3(kTileSlots), args,
-                                     kSolveTile, st);
+                                     (size_t)V.cap * 16, st);
 }
 
 void launch_apply_dp(const DevParams& P, const PassArgs& a, cudaStream_t st) {

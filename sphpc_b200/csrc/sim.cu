@@ -110,7 +110,7 @@ class DeviceSim {
   // transfers run at full link speed); released in release()
   std::vector<void*> pinned;
   bool nbr_valid = false;
-  int solve_max[6] = {-1, -1, -1, -1, -1, -1};  // solve_max_particles by kernel; -1: not asked
+  int sms = 1;
   uint32_t* crowded = nullptr;   // page-locked: set by the device (launch_count_cells)
 
   MlpState mlp{};
@@ -351,6 +351,7 @@ class DeviceSim {
     v.cstart = cstart;
     v.tiles = tiles;
     v.err = small + 2;
+    v.cap = tile_cap(n, sms);
     v.n = n;
     v.nx = nx; v.ny = ny; v.nz = nz;
     v.nxny = (uint32_t)nx * (uint32_t)ny;
@@ -827,9 +828,7 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
   bool fused_velocity = false;
   if (!adaptive && !collect && !carry_mode && !ready && iters == 0 && plain_cap > 0 &&
       plain_cap <= kSolveIterations) {
-    const int variant = (P.has_sdf ? 3 : 0) + (P.scorr_k == 0.0f ? 0 : P.scorr_n == 4 ? 1 : 2);
-    if (solve_max[variant] < 0) solve_max[variant] = solve_max_particles(P, device);
-    if (n > 0 && n <= solve_max[variant]) {
+    if (solve_fits(P, V, device, sms)) {
       Scope sc(this, "solve");
       SolveArgs sa{pd, pd_alt, nr, nr_alt, rho, vel, plain_cap, {}};
       for (int k = 0; k < plain_cap; ++k) sa.stiffness[k] = stiffness_of(solver.stiffness_k, k);
@@ -1141,6 +1140,7 @@ static int enter_data(Particles* particles, const Params* params, bool whole_pag
   }
   DeviceSim* s = new DeviceSim();
   cudaGetDevice(&s->device);
+  cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
   s->solver = current_solver();
   s->rho0 = particles->rest_density;
   s->mass = particles->rest_mass;

@@ -186,15 +186,39 @@ struct DevParams {
 // + dy nx, so it covers cells cx-1 .. cx+1 of that row for every slot of the
 // block, also where the block runs over the end of a row of cells.  Range r
 // starts at slot s[r] and at record o[r] of the tile that holds all nine one
-// after the other (total records; -1: more than kTileCap, or a particle whose
+// after the other (total records; -1: more than tile_cap, or a particle whose
 // neighbour cells are not the regular ones: the block's lists hold slots).
 // Range starts and lengths are even, so that pairs of slots stay together.
 //
-// kTileCap: nine ranges of 128 slots and about four cells at the ends hold 1400
-// records at the rest density; 1472 records of 16 bytes leave room for nine
-// blocks per SM.
+// tile_cap, the most records of a tile: nine ranges of 128 slots and about four
+// cells at the ends hold 1400 records at the rest density, and 1472 records of 16
+// bytes leave room for nine blocks per SM.  Where the fluid is pressed or its rows
+// are short some blocks need more (34% of 4096 particles 800 steps after a dam
+// break, 21% of 290k), and one that has no tile holds the others up when all run
+// at once: a set of up to four blocks per SM has the room that its passes over
+// two arrays leave a block.
+// A step of 4096 particles 115 -> 105 us, of 13,824 125 -> 107, of 32,768 138 ->
+// 120, of 68,921 172 -> 167.  In larger sets occupancy is worth more: with 1744
+// records 290k take 524 us for 534, 4.2M 5094 for 4982.
+// Entries are 16-bit byte offsets, and the build adds up to 32 records to one.
 constexpr int kTileSlots = 128;
 constexpr int kTileCap = 1472;
+constexpr int kTileCapMost = 4056;
+inline int tile_cap(int n, int sms) {
+  const int blocks = (n + kTileSlots - 1) / kTileSlots;
+  const int per_sm = blocks > sms ? (blocks + sms - 1) / sms : 1;
+  if (per_sm > 4) return kTileCap;
+  const int room = ((226 * 1024 / per_sm - 2048) / 32) & ~7;
+  return room < kTileCapMost ? room : kTileCapMost;
+}
+// Shared memory beyond 48 KB has to be allowed for a kernel: up to two of the
+// largest tiles, whatever this launch needs.
+template <class K>
+inline void allow_shared(K* kernel, size_t bytes) {
+  if (bytes > 48 * 1024)
+    cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kTileCapMost * 16);
+}
 struct TileInfo {
   int s[9], o[9], total, pad;
 };
@@ -207,6 +231,7 @@ struct NbrView {
   const TileInfo* __restrict__ tiles;   // [ceil(n / kTileSlots)]
   uint32_t* err;
   int n;
+  int cap;                              // records of a tile, at most (tile_cap)
   int nx, ny, nz;
   uint32_t nxny;
   int bx, by;
@@ -287,7 +312,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 // The tile of a block of kTileSlots threads: tile_load starts the copies of
-// NARR arrays of 16-byte records (array k at byte k * kTileCap * 16 of `tile`)
+// NARR arrays of 16-byte records (array k at byte k * cap * 16 of `tile`)
 // and returns whether the block has a tile; tile_wait waits for them.  Every
 // thread of the block calls both.
 template <int NARR>
@@ -312,7 +337,7 @@ __device__ __forceinline__ bool tile_load(const NbrView& v, const void* a0, cons
       const uint32_t bytes = (uint32_t)(e - o) * 16u;
       bulk_load(tile + o * 16, static_cast<const uint4*>(a0) + s, bytes, mbar);
       if (NARR == 2)
-        bulk_load(tile + (kTileCap + o) * 16, static_cast<const uint4*>(a1) + s, bytes, mbar);
+        bulk_load(tile + (v.cap + o) * 16, static_cast<const uint4*>(a1) + s, bytes, mbar);
     }
   }
   return total >= 0;
@@ -348,13 +373,14 @@ __device__ __forceinline__ void visit(const NbrView& v, bool tiled, const unsign
                                       const uint4* nr, const float4* __restrict__ e,
                                       int p, int cnt, uint4 blk, F&& f) {
   if (tiled) {
+    const unsigned char* tile_e = tile + v.cap * 16;
     auto load = [&](uint32_t w0, uint32_t w1) {
       const uint32_t o[4] = {w0 & 0xffffu, w0 >> 16, w1 & 0xffffu, w1 >> 16};
       Batch<NARR> b;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         b.r[u] = *reinterpret_cast<const uint4*>(tile + o[u]);
-        if (NARR == 2) b.e[u] = *reinterpret_cast<const float4*>(tile + kTileCap * 16 + o[u]);
+        if (NARR == 2) b.e[u] = *reinterpret_cast<const float4*>(tile_e + o[u]);
       }
       return b;
     };

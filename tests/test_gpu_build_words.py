@@ -30,6 +30,12 @@ def scene(tmp_path, dims):
     ((4, 4, 90), (1.0, 1.0, 0.25)),      # one tile; many short rows
     ((90, 5, 4), (0.2, 1.5, 1.5)),       # no tile; rows of about 40, few hits each
     ((31, 31, 31), (0.4, 1.3, 1.3)),     # no tile in the middle
+    # the room of a tile by the blocks an SM: 4056, 3552, 2344 and 1744 records
+    ((15, 16, 16), (0.45, 0.45, 0.45)),
+    ((15, 16, 16), (0.6, 0.6, 0.6)),
+    ((26, 26, 26), (0.62, 0.62, 0.62)),
+    ((38, 38, 38), (0.7, 0.7, 0.7)),
+    ((42, 42, 42), (0.85, 0.85, 0.85)),
 ])
 def test_buckets_of_dense_rows(tmp_path, dims, scale):
     with scene(tmp_path, dims) as sim:
