@@ -1104,9 +1104,9 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// Fields that AllocInitParticles lays on whole pages: position, velocity and
-// density (a frame's and a state's), from this size on.
-constexpr int kStateFields = 7;
+// Fields that AllocInitParticles lays on whole pages: position and density (a
+// frame's), from this size on.
+constexpr int kFrameFields = 4;
 constexpr size_t kLockBytes = (size_t)2 << 20;
 
 // A zeroed host array of n doubles, for free().  From 2 MB on it starts on a 2 MB
@@ -1124,7 +1124,7 @@ static double* host_array(size_t n) {
   return (double*)p;
 }
 
-// whole_pages: the host arrays of the first kStateFields fields come from
+// whole_pages: the host arrays of the first kFrameFields fields come from
 // host_array.
 static int enter_data(Particles* particles, const Params* params, bool whole_pages) {
   if (!particles || !params) return set_error(SPHPC_EINVAL, "sphpc_enter_data: null argument");
@@ -1150,19 +1150,19 @@ static int enter_data(Particles* particles, const Params* params, bool whole_pag
     // speed (15 MB to the host: 762 us pageable, 286 us locked).  Arrays of 64 MB
     // and more: all of them, the reference's calloc'd ones too.  Smaller ones may
     // share pages with other allocations and are left pageable, except those
-    // that AllocInitParticles laid on whole pages: the fields of a frame and of a
-    // state, from kLockBytes on (locking costs 0.35 ms an array and more, for 97k
-    // particles 5 ms a set against 0.3 ms a read-back of the state).  An array that the driver refuses stays
+    // that AllocInitParticles laid on whole pages: the fields of a frame, from
+    // kLockBytes on (locking costs 0.35 ms an array and more, for 97k particles
+    // 5 ms a set against 0.3 ms a read-back).  An array that the driver refuses stays
     // pageable.
     const size_t bytes = sizeof(double) * (size_t)particles->max_local;
     if (bytes >= ((size_t)64 << 20) || (whole_pages && bytes >= kLockBytes)) {
-      double* fields[20] = {particles->x, particles->y, particles->z, particles->v_x,
-                            particles->v_y, particles->v_z, particles->density, particles->x_star,
+      double* fields[20] = {particles->x, particles->y, particles->z, particles->density,
+                            particles->v_x, particles->v_y, particles->v_z, particles->x_star,
                             particles->y_star, particles->z_star, particles->dp_x, particles->dp_y,
                             particles->dp_z, particles->w_x, particles->w_y, particles->w_z,
                             particles->color_x, particles->color_y, particles->color_z,
                             particles->lambda};
-      const int count = bytes >= ((size_t)64 << 20) ? 20 : kStateFields;
+      const int count = bytes >= ((size_t)64 << 20) ? 20 : kFrameFields;
       for (int k = 0; k < count; ++k) {
         if (!fields[k]) continue;
         if (cudaHostRegister(fields[k], bytes, cudaHostRegisterDefault) == cudaSuccess)
@@ -1377,10 +1377,9 @@ int AllocInitParticles(struct Particles* particles, struct Params* params,
                           &particles->density, &particles->lambda};
   const bool large = n * sizeof(double) >= ((size_t)64 << 20);
   for (auto f : dfields) {
-    const bool state = f == &particles->x || f == &particles->y || f == &particles->z ||
-                       f == &particles->v_x || f == &particles->v_y || f == &particles->v_z ||
+    const bool frame = f == &particles->x || f == &particles->y || f == &particles->z ||
                        f == &particles->density;
-    *f = large || state ? host_array(n) : (double*)calloc(n, sizeof(double));
+    *f = large || frame ? host_array(n) : (double*)calloc(n, sizeof(double));
     if (!*f) return set_error(SPHPC_ENOMEM, "AllocInitParticles: calloc of %zu doubles", n);
   }
   particles->id = (int*)calloc(n, sizeof(int));
