@@ -311,17 +311,21 @@ __global__ void __launch_bounds__(kDistWarps * 32)
   if (live && warp == 0) phi[((long long)k * g.nj + j) * g.ni + i] = sqrtf(best);
 }
 
-// Sign of (b - a) x (p - a) in the (y, z) plane at the row (y, z) moved by an
-// infinitesimal (e, e^2), so that a row through an edge or a corner lies on one
-// side of it, the same for every triangle there.  The differences and products
-// of FP32 coordinates are exact in FP64 for coordinates within 2^29 of one
-// another, so opposite edges have opposite signs.
-__device__ __forceinline__ bool left_of(double ay, double az, double by, double bz, double y,
-                                        double z) {
-  const double ey = by - ay, ez = bz - az;
-  const double d = ey * (z - az) - ez * (y - ay);
-  if (d != 0.0) return d > 0.0;
-  return ez != 0.0 ? ez < 0.0 : ey > 0.0;
+// The part of edge a -> b in the winding number, in the (y, z) plane, of a triangle
+// about the row (y, z): +-1 where the ray from the row towards +y crosses the
+// edge, by the direction in which the triangle walks it.  The edge holds its lower
+// end and not its upper one, so a row through a corner crosses one of the edges
+// that pass it; the side is computed from the lower end whichever way the edge is
+// walked, by spelled-out operations.  So the two triangles of an edge always add
+// opposite parts, whatever rounds, and the crossings of a closed mesh with a row
+// add up to zero.
+__device__ __forceinline__ int edge_part(const float3& a, const float3& b, double y, double z) {
+  const bool below_a = a.z <= z, below_b = b.z <= z;
+  if (below_a == below_b) return 0;
+  const float3 u = below_a ? a : b, v = below_a ? b : a;
+  const double ey = __dsub_rn(v.y, u.y), ez = __dsub_rn(v.z, u.z);
+  const double side = __dsub_rn(__dmul_rn(ey, __dsub_rn(z, u.z)), __dmul_rn(ez, __dsub_rn(y, u.y)));
+  return side > 0.0 ? (below_a ? 1 : -1) : 0;
 }
 
 // Crossings of a closed mesh with the rows of samples along x: each triangle
@@ -338,31 +342,35 @@ __global__ void __launch_bounds__(kSdfBlock)
   if (t >= nt) return;
   const float3 a = corners[3 * (size_t)t], b = corners[3 * (size_t)t + 1],
                c = corners[3 * (size_t)t + 2];
+  const double xlo = fmin(fmin((double)a.x, b.x), c.x), xhi = fmax(fmax((double)a.x, b.x), c.x);
   const double ylo = fmin(fmin((double)a.y, b.y), c.y), yhi = fmax(fmax((double)a.y, b.y), c.y);
   const double zlo = fmin(fmin((double)a.z, b.z), c.z), zhi = fmax(fmax((double)a.z, b.z), c.z);
-  // one row more on each side: the samples' coordinates are rounded to FP32
+  // one row more on each side, and what rounding to FP32 moves a sample's coordinate
   auto clip = [](double v, int n) { return (int)fmin(fmax(v, 0.0), (double)n); };
-  const int j0 = clip(floor((ylo - g.oy) / g.dx) - 1, g.nj), j1 = clip(ceil((yhi - g.oy) / g.dx) + 2, g.nj);
-  const int k0 = clip(floor((zlo - g.oz) / g.dx) - 1, g.nk), k1 = clip(ceil((zhi - g.oz) / g.dx) + 2, g.nk);
+  const double ym = 0x1p-23 * fmax(fabs(ylo), fabs(yhi)), zm = 0x1p-23 * fmax(fabs(zlo), fabs(zhi));
+  const int j0 = clip(floor((ylo - ym - g.oy) / g.dx) - 1, g.nj),
+            j1 = clip(ceil((yhi + ym - g.oy) / g.dx) + 2, g.nj),
+            k0 = clip(floor((zlo - zm - g.oz) / g.dx) - 1, g.nk),
+            k1 = clip(ceil((zhi + zm - g.oz) / g.dx) + 2, g.nk);
   const int nj = j1 - j0;
   if (nj <= 0 || k1 <= k0) return;
   for (long long r = lane; r < (long long)nj * (k1 - k0); r += 32) {
     const int j = j0 + (int)(r % nj), k = k0 + (int)(r / nj);
     const float3 s = sample_pos(g, 0, j, k);
-    const bool l0 = left_of(a.y, a.z, b.y, b.z, s.y, s.z), l1 = left_of(b.y, b.z, c.y, c.z, s.y, s.z),
-               l2 = left_of(c.y, c.z, a.y, a.z, s.y, s.z);
-    if (l0 != l1 || l1 != l2) continue;
-    // the plane through the triangle at (y, z)
+    const int wind = edge_part(a, b, s.y, s.z) + edge_part(b, c, s.y, s.z) + edge_part(c, a, s.y, s.z);
+    if (wind == 0) continue;
+    // the plane through the triangle at (y, z), within the triangle's range (also
+    // where rounding leaves no normal along x)
     const double ux = (double)b.x - a.x, uy = (double)b.y - a.y, uz = (double)b.z - a.z;
     const double vx = (double)c.x - a.x, vy = (double)c.y - a.y, vz = (double)c.z - a.z;
     const double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
-    if (nx == 0.0) continue;
-    const double x = a.x - (ny * ((double)s.y - a.y) + nz * ((double)s.z - a.z)) / nx;
+    const double plane = a.x - (ny * ((double)s.y - a.y) + nz * ((double)s.z - a.z)) / nx;
+    const double x = fmin(fmax(plane, xlo), xhi);
     int i = (int)fmin(fmax(ceil((x - g.ox) / g.dx), 0.0), (double)g.ni);
     while (i > 0 && (double)sample_pos(g, i - 1, j, k).x > x) --i;
     while (i < g.ni && (double)sample_pos(g, i, j, k).x <= x) ++i;
     // walking +x, the winding number drops by one where the normal points to +x
-    if (i < g.ni) atomicAdd(step + ((long long)k * g.nj + j) * g.ni + i, l0 ? -1 : 1);
+    if (i < g.ni) atomicAdd(step + ((long long)k * g.nj + j) * g.ni + i, -wind);
   }
 }
 
