@@ -944,7 +944,7 @@ int launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint
     return 0;
   }
   if (ncells <= kBoundsMaxCells) {
-    launch_bounds(keys_sorted, n, (int)ncells + 1, cstart, false, st);
+    launch_bounds(keys_sorted, n, (int)ncells + 1, cstart, false, st, err);
     return 1;
   }
   cudaMemsetAsync(gap_count, 0, sizeof(uint32_t), st);

@@ -253,12 +253,15 @@ __device__ int warp_lower_bound(const uint32_t* __restrict__ keys, int n, int64_
 // kBoundRange keys is searched cell by cell instead.  Bounds: the latency of the
 // two searches (four dependent loads at 1M keys).  1.8M cells over 1M keys, cold
 // caches: 38 us with a binary search of all keys per cell, 20 us so.
+// Keys that are out of order give wrong starts, all of them in [0, n].  With err,
+// the cells are all that there are (the last one ends the table), and a key beyond
+// them or out of its block's cells raises its bit.
 constexpr int kBoundPer = 8;
 constexpr int kBoundCells = 256 * kBoundPer;
 constexpr int kBoundRange = 1 << 15;
 __global__ void __launch_bounds__(256)
     k_bounds(const uint32_t* __restrict__ keys, int n, int count, int first,
-             uint32_t* __restrict__ out) {
+             uint32_t* __restrict__ out, uint32_t* __restrict__ err) {
   __shared__ int s_first[kBoundCells];
   __shared__ int s_range[2], s_min[8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -272,6 +275,9 @@ __global__ void __launch_bounds__(256)
   for (int i = t; i < kBoundCells; i += 256) s_first[i] = INT_MAX;
   __syncthreads();
   const int lo = s_range[0], hi = s_range[1];
+  // (the start of the table's last cell)
+  if (err && t == 0 && c0 + nc == count && n > 0 && (int64_t)__ldg(keys + n - 1) >= count - 1)
+    atomicOr(err, 4u);  // kErrCellRange
   if (hi - lo > kBoundRange) {
     for (int i = t; i < nc; i += 256) {
       int a = lo, b = hi;
@@ -285,7 +291,12 @@ __global__ void __launch_bounds__(256)
   }
   for (int j = lo + t; j < hi; j += 256) {
     const uint32_t k = __ldg(keys + j);
-    if (j == lo || __ldg(keys + j - 1) != k) s_first[(int64_t)k - v0] = j;
+    const int64_t c = (int64_t)k - v0;
+    if (c < 0 || c >= nc) {
+      if (err) atomicOr(err, 4u);  // kErrCellRange
+    } else if (j == lo || __ldg(keys + j - 1) != k) {
+      s_first[c] = j;
+    }
   }
   __syncthreads();
   // suffix minimum: kBoundPer cells per thread, then over the lanes and the warps
@@ -428,11 +439,11 @@ cudaError_t lookback_wait_probe(int spin_limit, uint32_t* err_bits) {
 }
 
 cudaError_t launch_bounds(const uint32_t* keys, int n, int count, uint32_t* out, bool upper,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, uint32_t* err) {
   if (count <= 0) return cudaSuccess;
   // the upper bound of c is the lower bound of c + 1
   const int blocks = (int)(((int64_t)count + kBoundCells - 1) / kBoundCells);
-  k_bounds<<<blocks, 256, 0, stream>>>(keys, n, count, upper ? 1 : 0, out);
+  k_bounds<<<blocks, 256, 0, stream>>>(keys, n, count, upper ? 1 : 0, out, err);
   return cudaGetLastError();
 }
 

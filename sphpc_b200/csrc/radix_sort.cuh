@@ -102,8 +102,9 @@ __device__ __forceinline__ void count_key_digits(uint32_t* s_hist, uint32_t key,
 cudaError_t lookback_wait_probe(int spin_limit, uint32_t* err_bits);
 
 // lower_bound / upper_bound of every c in [0, count) over sorted keys
-// (FindLowerBounds / FindUpperBounds, thrust_c.cu:93-120).
+// (FindLowerBounds / FindUpperBounds, thrust_c.cu:93-120).  err: the table of
+// all cells, ended by c = count - 1; keys not below that raise kErrCellRange.
 cudaError_t launch_bounds(const uint32_t* keys, int n, int count, uint32_t* out, bool upper,
-                          cudaStream_t stream);
+                          cudaStream_t stream, uint32_t* err = nullptr);
 
 }  // namespace sphpc
