@@ -95,7 +95,6 @@ class DeviceSim {
   float4 *color_alt = nullptr, *omega_alt = nullptr, *dp_alt = nullptr;
   float *rho_alt = nullptr, *lam_alt = nullptr;
   uint32_t *ids = nullptr, *ids_spare = nullptr, *keys_by_id = nullptr, *loc_by_id = nullptr;
-  uint32_t* keys_sorted = nullptr;  // view into keys_by_id or sort.keys_alt; null: not made
   uint32_t *cellp = nullptr, *nbr = nullptr, *cstart = nullptr;
   float4* xsa = nullptr;
   TileInfo* tiles = nullptr;  // of the current lists
@@ -601,7 +600,6 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
                                    sort.vals_alt, predict, crowded, err(), stream);
     R = ids_spare;
     order = SlotOrder{sort.keys_alt, sort.vals_alt, keys_by_id, cstart, R};
-    keys_sorted = nullptr;
   } else {
     uint32_t* K = nullptr;
     {
@@ -619,7 +617,6 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
         return set_error(SPHPC_ECUDA, "radix sort: %s", cudaGetErrorString(e));
       launches += (unsigned)passes;
     }
-    keys_sorted = K;
     {
       Scope sc(this, "cell_starts");
       launches += launch_cell_starts(K, n, C, cstart, gaps, gap_count(), err(), stream);
@@ -1492,13 +1489,14 @@ int sphpc_get_cell_data(const struct Particles* particles, unsigned int* hash_va
                         unsigned int* particle_ids, unsigned int* start_indices) {
   SPHPC_SIM(s, particles);
   if (!s->nbr_valid) return set_error(SPHPC_ENOTREADY, "no cell data yet");
-  if (hash_values && !s->keys_sorted) {
-    s->keys_sorted = s->sort.keys_alt;
-    launch_slot_keys(s->cstart, s->C, s->keys_sorted, s->stream);
+  if (hash_values) {
+    // from the cell starts on every query: the build's keys lie in buffers that the
+    // next one writes, and a recorded build runs without this side seeing it
+    uint32_t* keys = s->sort.keys_alt;
+    launch_slot_keys(s->cstart, s->C, keys, s->stream);
+    SPHPC_CK(cudaMemcpyAsync(hash_values, keys, sizeof(uint32_t) * s->n, cudaMemcpyDeviceToHost,
+                             s->stream));
   }
-  if (hash_values)
-    SPHPC_CK(cudaMemcpyAsync(hash_values, s->keys_sorted, sizeof(uint32_t) * s->n,
-                             cudaMemcpyDeviceToHost, s->stream));
   if (particle_ids)
     SPHPC_CK(cudaMemcpyAsync(particle_ids, s->ids, sizeof(uint32_t) * s->n,
                              cudaMemcpyDeviceToHost, s->stream));
@@ -1787,7 +1785,6 @@ int sphpc_slab_unpack(struct Particles* particles, const void* recv_left, int co
   s->nbr_valid = false;
   s->have_carry = false;
   s->prev_err0 = -1.0;
-  s->keys_sorted = nullptr;
   uint32_t herr = 0;
   SPHPC_CK(cudaMemcpy(&herr, s->sort.err, sizeof(uint32_t), cudaMemcpyDeviceToHost));
   if (herr) return set_error(SPHPC_EKERNEL, "sphpc_slab_unpack: sort error bits 0x%x", herr);
