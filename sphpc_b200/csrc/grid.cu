@@ -134,12 +134,16 @@ __global__ void __launch_bounds__(kBlock)
 // 4096: 42 and 27.  Empty cells cost 12 bytes each here and 4 there: at 27 cells a
 // particle 182 us against 229 (1M particles), 64 against 98 (262k).
 //
-// The rank by comparing takes time with the square of a cell's particles: 262,144
-// in eight cells are ranked in 12.7 ms, in digit passes in 65 us.  A cell of more
-// than kCrowded sets *crowded, host memory, and the set goes over to the digit
-// passes when the host sees it; the slots are the same either way.
+// The rank by comparing takes time with the square of a cell's particles, so a
+// cell of more than kCrowded is put in order instead, by the block that places its
+// last particle (order_cell), and sets *crowded, host memory: digit passes are faster for
+// such a set, and it goes over to them when the host sees it; the slots are the
+// same either way.  Where the line lies, us from hash to reorder with 256 / 512 / 1000
+// particles a cell, ranked by comparing and by digit passes: 32,768 particles 31 / 32 /
+// 41 and 74 / 69 / 69; 262,144 48 / 59 / 83 and 96 / 96 / 80; 1,048,576 111 / 153 / 222 and
+// 161 / 141 / 141; 4.2M 348 / 507 by comparing, 359 by digits (their build takes 8 ms).
 // ---------------------------------------------------------------------------
-constexpr uint32_t kCrowded = 1024;
+constexpr uint32_t kCrowded = 512;
 
 // keys[i] of slot i, and its rank among its cell's particles in the order that
 // the atomics happen to take.  The lanes of a cell share one atomic: eight
@@ -180,7 +184,8 @@ __device__ __forceinline__ void st_state(unsigned long long* p, unsigned long lo
 
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_counts(uint32_t* __restrict__ cells, uint32_t m, unsigned long long* __restrict__ state,
-                  volatile uint32_t* crowded, uint32_t* __restrict__ err) {
+                  volatile uint32_t* crowded, uint32_t* __restrict__ any_crowded,
+                  uint32_t* __restrict__ err) {
   __shared__ uint32_t s_warp[kScanThreads / 32];
   __shared__ uint32_t s_block, s_before;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -211,7 +216,7 @@ __global__ void __launch_bounds__(kScanThreads)
     v[u] = sum;
     sum += x;
   }
-  if (most > kCrowded) *crowded = 1u;
+  if (most > kCrowded) *any_crowded = *crowded = 1u;
   uint32_t upto = sum;
 #pragma unroll
   for (int k = 1; k < 32; k <<= 1) {
@@ -271,16 +276,131 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// Id and old slot of every particle into its cell's range.
-__global__ void __launch_bounds__(kBlock)
-    k_place(int n, const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ keys,
-            const uint32_t* __restrict__ rank, const uint32_t* __restrict__ ids,
-            uint32_t* __restrict__ cell_ids, uint32_t* __restrict__ cell_src) {
+// The m ids of one cell into ascending order, their old slots with them, by one
+// block: digit passes from the lowest digit on, between the cell's range of ids and
+// src and that of ids2 and src2 (an even number, so that they end in the first).
+// One block takes about 3 ns a pair and pass: 3.1 ms for 262,144 particles in one
+// cell, 55 ms for 4.2M (by comparing 12.7 ms, and 256 times that).  Steps that were
+// launched before the host saw the cell pay it, those after it go by digit passes.
+constexpr int kOrderItems = 8;
+__device__ __noinline__ void order_cell(uint32_t* ids, uint32_t* src, uint32_t* ids2,
+                                        uint32_t* src2, uint32_t m, int passes) {
+  __shared__ uint32_t s_base[kRadix], s_sum[kBlock / 32];
+  __shared__ uint32_t s_warp[kBlock / 32][kRadix + 1];
+  static_assert(kBlock == kRadix, "a thread a digit");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int pass = 0; pass < passes; ++pass) {
+    const int shift = pass * kRadixBits;
+    s_base[t] = 0;
+    __syncthreads();
+    for (uint32_t i = t; i < m; i += kBlock)
+      atomicAdd(&s_base[(__ldcg(ids + i) >> shift) & (kRadix - 1)], 1u);
+    __syncthreads();
+    const uint32_t all = s_base[t];
+    uint32_t upto = all;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, k);
+      if (lane >= k) upto += y;
+    }
+    if (lane == 31) s_sum[warp] = upto;
+    __syncthreads();
+    uint32_t first = upto - all;
+    for (int w = 0; w < warp; ++w) first += s_sum[w];
+    s_base[t] = first;
+    for (uint32_t t0 = 0; t0 < m; t0 += kBlock * kOrderItems) {
+      for (int k = t; k < kBlock / 32 * (kRadix + 1); k += kBlock) (&s_warp[0][0])[k] = 0;
+      __syncthreads();
+      uint32_t id[kOrderItems], rank[kOrderItems];
+#pragma unroll
+      for (int u = 0; u < kOrderItems; ++u) {
+        const uint32_t i = t0 + (warp * kOrderItems + u) * 32 + lane;
+        id[u] = i < m ? __ldcg(ids + i) : 0u;
+        const uint32_t d = i < m ? (id[u] >> shift) & (kRadix - 1) : (uint32_t)kRadix;
+        const unsigned same = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = s_warp[warp][d];
+        __syncwarp();
+        rank[u] = before + __popc(same & ((1u << lane) - 1u));
+        if (lane == __ffs((int)same) - 1) s_warp[warp][d] = before + __popc(same);
+        __syncwarp();
+      }
+      __syncthreads();
+      uint32_t at = s_base[t];
+      for (int w = 0; w < kBlock / 32; ++w) {
+        const uint32_t c = s_warp[w][t];
+        s_warp[w][t] = at;
+        at += c;
+      }
+      s_base[t] = at;
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kOrderItems; ++u) {
+        const uint32_t i = t0 + (warp * kOrderItems + u) * 32 + lane;
+        if (i >= m) continue;
+        const uint32_t to = s_warp[warp][(id[u] >> shift) & (kRadix - 1)] + rank[u];
+        ids2[to] = id[u];
+        src2[to] = __ldcg(src + i);
+      }
+      __syncthreads();
+    }
+    uint32_t* x = ids;
+    ids = ids2;
+    ids2 = x;
+    x = src;
+    src = src2;
+    src2 = x;
+  }
+}
+
+// Id and old slot of every particle into its cell's range.  With a crowded cell
+// about (`any`), the threads count what they have placed of it in `placed`, a word for
+// every kCrowded + 1 slots: no two crowded cells start in the same ones.  The block
+// with the last particle of a cell puts it in order.
+struct PlaceArgs {
+  const uint32_t *keys, *rank, *ids, *any;
+  uint32_t *placed;
+  uint32_t *cell_ids, *cell_src;  // written by all blocks and read by one
+  uint32_t *ids2, *src2;          // scratch
+  int passes;                     // digit passes that order ids
+};
+__global__ void __launch_bounds__(kBlock, 8)
+    k_place(int n, const uint32_t* __restrict__ cstart, const PlaceArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t j = min(__ldg(cstart + __ldg(keys + i)) + __ldg(rank + i), (uint32_t)n - 1u);
-  cell_ids[j] = __ldg(ids + i);
-  cell_src[j] = (uint32_t)i;
+  const bool any = __ldg(a.any) != 0;
+  uint32_t key = 0, b = 0;
+  if (i < n) {
+    key = __ldg(a.keys + i);
+    b = __ldg(cstart + key);
+    const uint32_t j = min(b + __ldg(a.rank + i), (uint32_t)n - 1u);
+    a.cell_ids[j] = __ldg(a.ids + i);
+    a.cell_src[j] = (uint32_t)i;
+  }
+  if (!any) return;
+  __shared__ uint32_t s_first[kBlock], s_count[kBlock];
+  __shared__ int s_cells;
+  if (threadIdx.x == 0) s_cells = 0;
+  __syncthreads();
+  const uint32_t m = i < n ? min(__ldg(cstart + key + 1), (uint32_t)n) - b : 0u;
+  const unsigned on = __ballot_sync(0xffffffffu, i < n && m > kCrowded && m <= (uint32_t)n);
+  if (on >> (threadIdx.x & 31) & 1u) {
+    const unsigned same = __match_any_sync(on, key);
+    __threadfence();
+    __syncwarp(same);
+    if ((int)(threadIdx.x & 31) == __ffs((int)same) - 1) {
+      const uint32_t here = (uint32_t)__popc(same);
+      if (atomicAdd(a.placed + b / (kCrowded + 1), here) + here == m) {
+        const int c = atomicAdd(&s_cells, 1);
+        s_first[c] = b;
+        s_count[c] = m;
+      }
+    }
+  }
+  __syncthreads();
+  __threadfence();
+  for (int c = 0; c < s_cells; ++c) {
+    const uint32_t f = s_first[c];
+    order_cell(a.cell_ids + f, a.cell_src + f, a.ids2 + f, a.src2 + f, s_count[c], a.passes);
+  }
 }
 
 // Keys of the slots from the cell starts.
@@ -305,9 +425,11 @@ __global__ void __launch_bounds__(kBlock)
     src = __ldg(o.src + j);
     const uint32_t key = __ldg(o.keys + src);
     const uint32_t b = __ldg(o.cstart + key), e = __ldg(o.cstart + key + 1);
-    uint32_t at = b;
-    for (uint32_t k = b; k < e; ++k) at += __ldg(o.ids + k) < id ? 1u : 0u;
-    j = (int)min(at, (uint32_t)P.n - 1u);
+    if (e - b <= kCrowded) {  // (a crowded cell's are in order)
+      uint32_t at = b;
+      for (uint32_t k = b; k < e; ++k) at += __ldg(o.ids + k) < id ? 1u : 0u;
+      j = (int)min(at, (uint32_t)P.n - 1u);
+    }
     o.ids_out[j] = id;
   } else {
     src = __ldg(o.src + id);
@@ -887,9 +1009,11 @@ void launch_hash(const DevParams& P, const PD* pd, const float4* vel, const uint
                                            passes, predict ? 1 : 0, err);
 }
 
-size_t cell_table_words(uint32_t ncells) {
-  // cstart[0..C], then the scan's ticket and block states
-  return (((size_t)ncells + 2) & ~(size_t)1) + 2 * (2 + (size_t)ncells / kScanItems + 1);
+size_t cell_table_words(uint32_t ncells, int cap) {
+  // cstart[0..C], then the scan's ticket and block states, then whether a cell is
+  // crowded and what is placed of the crowded ones
+  return (((size_t)ncells + 2) & ~(size_t)1) + 2 * (2 + (size_t)ncells / kScanItems + 1) + 1 +
+         (size_t)cap / (kCrowded + 1) + 1;
 }
 
 bool counts_cells(int n, uint32_t ncells) {
@@ -897,17 +1021,21 @@ bool counts_cells(int n, uint32_t ncells) {
 }
 
 int launch_count_cells(const DevParams& P, const PD* pd, const float4* vel, const uint32_t* ids,
-                       uint32_t* cstart, uint32_t* keys, uint32_t* rank, uint32_t* cell_ids,
-                       uint32_t* cell_src, bool predict, uint32_t* crowded, uint32_t* err,
-                       cudaStream_t st) {
+                       uint32_t* cstart, const CountScratch& s, bool predict, uint32_t* crowded,
+                       uint32_t* err, cudaStream_t st) {
   const uint32_t m = P.ncells + 1;
-  unsigned long long* state =
-      reinterpret_cast<unsigned long long*>(cstart + (((size_t)P.ncells + 2) & ~(size_t)1));
-  cudaMemsetAsync(cstart, 0, cell_table_words(P.ncells) * sizeof(uint32_t), st);
-  k_count<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, vel, keys, rank, cstart, predict ? 1 : 0, err);
+  uint32_t* after = cstart + (((size_t)P.ncells + 2) & ~(size_t)1);
+  unsigned long long* state = reinterpret_cast<unsigned long long*>(after);
+  uint32_t* any = after + 2 * (2 + (size_t)P.ncells / kScanItems + 1);
+  cudaMemsetAsync(cstart, 0, cell_table_words(P.ncells, P.n) * sizeof(uint32_t), st);
+  k_count<<<grid_for(P.n), kBlock, 0, st>>>(P, pd, vel, s.keys, s.rank, cstart, predict ? 1 : 0,
+                                            err);
   k_scan_counts<<<(int)(((uint64_t)m + kScanItems - 1) / kScanItems), kScanThreads, 0, st>>>(
-      cstart, m, state, crowded, err);
-  k_place<<<grid_for(P.n), kBlock, 0, st>>>(P.n, cstart, keys, rank, ids, cell_ids, cell_src);
+      cstart, m, state, crowded, any, err);
+  int passes = 2;  // digits of the ids below n, an even number
+  while (passes < 4 && (uint64_t)P.n > 1ull << (passes * kRadixBits)) passes += 2;
+  const PlaceArgs a{s.keys, s.rank, ids, any, any + 1, s.cell_ids, s.cell_src, s.ids2, s.src2, passes};
+  k_place<<<grid_for(P.n), kBlock, 0, st>>>(P.n, cstart, a);
   return 3;
 }
 

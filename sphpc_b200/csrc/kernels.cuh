@@ -27,16 +27,19 @@ void launch_hash(const DevParams& P, const PD* pd, const float4* vel, const uint
 
 // The same by counting, for grids of up to 32 cells a particle
 // (counts_cells): the keys in slot order, the cell start table, and every
-// particle's id and old slot somewhere in its cell's range (cell_ids, cell_src).
-// cstart has cell_table_words(C) words; rank is scratch; *crowded (host memory)
-// becomes 1 when a cell holds so many that digit passes are faster.  Returns the kernels
-// launched.
-size_t cell_table_words(uint32_t ncells);
+// particle's id and old slot somewhere in its cell's range (cell_ids, cell_src; in
+// the order of the ids where the cell is crowded).  cstart has
+// cell_table_words(C, n or more) words; rank, ids2 and src2 are scratch of n words;
+// *crowded (host memory) becomes 1 when a cell holds so many that digit passes are
+// faster.  Returns the kernels launched.
+struct CountScratch {
+  uint32_t *keys, *rank, *cell_ids, *cell_src, *ids2, *src2;
+};
+size_t cell_table_words(uint32_t ncells, int cap);
 bool counts_cells(int n, uint32_t ncells);
 int launch_count_cells(const DevParams& P, const PD* pd, const float4* vel, const uint32_t* ids,
-                       uint32_t* cstart, uint32_t* keys, uint32_t* rank, uint32_t* cell_ids,
-                       uint32_t* cell_src, bool predict, uint32_t* crowded, uint32_t* err,
-                       cudaStream_t st);
+                       uint32_t* cstart, const CountScratch& s, bool predict, uint32_t* crowded,
+                       uint32_t* err, cudaStream_t st);
 // keys[j] of every slot from the cell start table.
 void launch_slot_keys(const uint32_t* cstart, uint32_t ncells, uint32_t* keys, cudaStream_t st);
 

@@ -111,6 +111,8 @@ class DeviceSim {
   bool nbr_valid = false;
   int sms = 1;
   uint32_t* crowded = nullptr;   // page-locked: set by the device (launch_count_cells)
+  uint32_t crowded_searches = 0; // by digit passes since then
+  static constexpr uint32_t kCrowdedSearches = 64;
 
   MlpState mlp{};
   uint4 *nr = nullptr, *nr_alt = nullptr;  // 16-byte neighbour records (x* fixed point, payload)
@@ -334,7 +336,7 @@ class DeviceSim {
     nx = nnx; ny = nny; nz = nnz; C = CC; bx = bxx; by = byy;
     passes = (bits_for(C - 1) + kRadixBits - 1) / kRadixBits;
     if (passes > kMaxPasses) passes = kMaxPasses;
-    SPHPC_RC(dalloc(&cstart, cell_table_words(C)));
+    SPHPC_RC(dalloc(&cstart, cell_table_words(C, cap)));
     dfree(gaps);
     SPHPC_RC(dalloc(&gaps, (size_t)cap + 4 + C / 4096));
     SPHPC_CK(cudaMemsetAsync(cstart, 0, sizeof(uint32_t) * ((size_t)C + 1), stream));
@@ -594,11 +596,18 @@ int DeviceSim::find_neighbors(const DevParams& P, bool predict, bool full, bool 
   if (full) SPHPC_RC(ensure_full_alts());
   SlotOrder order{};
   uint32_t* R = nullptr;
-  if (counts_cells(n, C) && !*static_cast<volatile uint32_t*>(crowded)) {
+  bool counted = counts_cells(n, C);
+  if (volatile uint32_t* seen = crowded; counted && *seen) {
+    // by digit passes for a while; then the set may have spread out again
+    counted = ++crowded_searches >= kCrowdedSearches;
+    if (counted) *seen = crowded_searches = 0;
+  }
+  if (counted) {
     Scope sc(this, "count_cells");
-    launches += launch_count_cells(P, pd, vel, ids, cstart, keys_by_id, loc_by_id, sort.keys_alt,
-                                   sort.vals_alt, predict, crowded, err(), stream);
     R = ids_spare;
+    // (cellp is free until the reorder writes it, the spare ids until they are these)
+    const CountScratch cs{keys_by_id, loc_by_id, sort.keys_alt, sort.vals_alt, R, cellp};
+    launches += launch_count_cells(P, pd, vel, ids, cstart, cs, predict, crowded, err(), stream);
     order = SlotOrder{sort.keys_alt, sort.vals_alt, keys_by_id, cstart, R};
   } else {
     uint32_t* K = nullptr;
