@@ -44,6 +44,16 @@ static int alloc_allowed(size_t bytes) {
   return SPHPC_OK;
 }
 
+// Cooperative launches still to be refused (sphpc_fail_solve_launch).
+static std::atomic<int> g_solve_fail_count{0};
+
+static bool solve_refused() {
+  int left = g_solve_fail_count.load();
+  while (left > 0 && !g_solve_fail_count.compare_exchange_weak(left, left - 1)) {
+  }
+  return left > 0;
+}
+
 template <class T>
 static int dalloc(T** p, size_t n) {
   if (n == 0) n = 1;
@@ -838,11 +848,20 @@ int DeviceSim::run_step(const DevParams& P, const Params& prm) {
       Scope sc(this, "solve");
       SolveArgs sa{pd, pd_alt, nr, nr_alt, rho, vel, plain_cap, {}};
       for (int k = 0; k < plain_cap; ++k) sa.stiffness[k] = stiffness_of(solver.stiffness_k, k);
-      SPHPC_CK(launch_solve(P, V, sa, stream));
-      launches += 1;
-      std::swap(pd, pd_alt);
-      iters = plain = plain_cap;
-      fused_velocity = true;
+      const cudaError_t e = solve_refused() ? cudaErrorCooperativeLaunchTooLarge
+                                            : launch_solve(P, V, sa, stream);
+      if (e == cudaSuccess) {
+        launches += 1;
+        std::swap(pd, pd_alt);
+        iters = plain = plain_cap;
+        fused_velocity = true;
+      } else if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported ||
+                 e == cudaErrorNotPermitted) {
+        // the stream has less than the device (a part of its SMs, a share): pass by pass
+        cudaGetLastError();
+      } else {
+        return set_error(SPHPC_ECUDA, "solve: %s", cudaGetErrorString(e));
+      }
     }
   }
   while (!converged && iters < plain_cap) {
@@ -2142,6 +2161,12 @@ static int wait_check(const char* what, cudaError_t e, uint32_t bits, unsigned i
 int sphpc_fail_device_alloc(int after) {
   if (after < -1) return set_error(SPHPC_EINVAL, "sphpc_fail_device_alloc: %d < -1", after);
   g_alloc_fail_after.store(after);
+  return SPHPC_OK;
+}
+
+int sphpc_fail_solve_launch(int count) {
+  if (count < 0) return set_error(SPHPC_EINVAL, "sphpc_fail_solve_launch: %d < 0", count);
+  g_solve_fail_count.store(count);
   return SPHPC_OK;
 }
 
