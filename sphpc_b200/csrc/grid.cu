@@ -553,13 +553,18 @@ __device__ __forceinline__ bool shifted_coord(double x, double h, int nmax, int&
   return true;
 }
 
+// Whether the walk visits the cells c-1, c, c+1 of an axis that the grid has, for a
+// particle in cell c.  A particle beyond the grid is not regular: its cell is the
+// last one, its key another's (key_of), and the rows of a block's tile are found
+// from both.
 __device__ __forceinline__ bool axis_regular(double x, double h, int c, int nmax) {
   int g;
+  const bool own = shifted_coord(x, h, nmax, g) && g == c;
   const bool vm = shifted_coord(__dadd_rn(x, -h), h, nmax, g);
   const bool okm = vm ? (g == c - 1) : (c == 0);
   const bool vp = shifted_coord(__dadd_rn(x, h), h, nmax, g);
   const bool okp = vp ? (g == c + 1) : (c == nmax - 1);
-  return okm && okp;
+  return own && okm && okp;
 }
 
 // r^2 < h^2 exactly as neighbors.c:278-285 evaluates it on the canonical
