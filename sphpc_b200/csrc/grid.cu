@@ -559,12 +559,12 @@ __device__ __forceinline__ bool shifted_coord(double x, double h, int nmax, int&
 // from both.
 __device__ __forceinline__ bool axis_regular(double x, double h, int c, int nmax) {
   int g;
-  const bool own = shifted_coord(x, h, nmax, g) && g == c;
+  if (c == nmax - 1 && !shifted_coord(x, h, nmax, g)) return false;
   const bool vm = shifted_coord(__dadd_rn(x, -h), h, nmax, g);
   const bool okm = vm ? (g == c - 1) : (c == 0);
   const bool vp = shifted_coord(__dadd_rn(x, h), h, nmax, g);
   const bool okp = vp ? (g == c + 1) : (c == nmax - 1);
-  return own && okm && okp;
+  return okm && okp;
 }
 
 // r^2 < h^2 exactly as neighbors.c:278-285 evaluates it on the canonical
@@ -1066,8 +1066,8 @@ void launch_reorder(const DevParams& P, const SlotOrder& order, const PD* pd_in,
 }
 
 // Up to kBoundsMaxCells cells the bounds kernel writes the table in one launch
-// (two blocks per SM and one wave); beyond, its search per 1024 cells costs
-// more than the worklist's second launch.
+// (256 blocks of 2048 cells, all resident at once); beyond, its two searches per
+// block cost more than the worklist's second launch.
 constexpr uint32_t kBoundsMaxCells = 1u << 19;
 
 int launch_cell_starts(const uint32_t* keys_sorted, int n, uint32_t ncells, uint32_t* cstart,

@@ -291,11 +291,10 @@ __global__ void __launch_bounds__(256)
   }
   for (int j = lo + t; j < hi; j += 256) {
     const uint32_t k = __ldg(keys + j);
-    const int64_t c = (int64_t)k - v0;
-    if (c < 0 || c >= nc) {
-      if (err) atomicOr(err, 4u);  // kErrCellRange
-    } else if (j == lo || __ldg(keys + j - 1) != k) {
-      s_first[c] = j;
+    if (j == lo || __ldg(keys + j - 1) != k) {
+      const uint32_t c = k - (uint32_t)v0;
+      if (c < (uint32_t)nc) s_first[c] = j;
+      else if (err) atomicOr(err, 4u);  // kErrCellRange
     }
   }
   __syncthreads();
